@@ -207,6 +207,8 @@ struct ffs_pool {
     int sms = 0;              // SMs of the device, queried at creation
     int grid_dense[kPoolNumShapes] = {};
     int grid_link = 0;        // resident CTAs of the link-cell kernel (one wave)
+    float *stage = nullptr;   // ffs_pool_get_moments' AoS copy of one episode, kept (at most the largest episode's size)
+    size_t stage_bytes = 0;
 };
 
 namespace {
@@ -498,7 +500,7 @@ ffs_status ffs_pool_destroy(ffs_pool *p)
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
     cudaFree(p->lt.keys); cudaFree(p->lt.links); cudaFree(p->lt.list); cudaFree(p->lt.count); cudaFree(p->owner);
-    cudaFree(p->d_eps); cudaFree(p->d_prm); cudaFree(p->d_act); cudaFree(p->d_out); cudaFree(p->arena_mem);
+    cudaFree(p->d_eps); cudaFree(p->d_prm); cudaFree(p->d_act); cudaFree(p->d_out); cudaFree(p->arena_mem); cudaFree(p->stage);
     for (int b = 0; b < 2; ++b)
         if (p->h_prm[b]) cudaFreeHost(p->h_prm[b]);
     if (p->h_act) cudaFreeHost(p->h_act);
@@ -771,8 +773,15 @@ ffs_status ffs_pool_get_moments(ffs_pool *p, int slot, float *moments)
     ffs_status r = wait_idle(p);
     if (r != FFS_OK) return r;
     const Slot &s = p->slots[slot];
-    float *stage = nullptr;
-    POOL_CK(cudaMalloc(&stage, sizeof(float) * 6 * (size_t)s.ncell));
+    const size_t bytes = sizeof(float) * 6 * (size_t)s.ncell;
+    if (p->stage_bytes < bytes) {
+        cudaFree(p->stage);
+        p->stage = nullptr;
+        p->stage_bytes = 0;
+        POOL_CK(cudaMalloc(&p->stage, bytes));
+        p->stage_bytes = bytes;
+    }
+    float *stage = p->stage;
     cudaError_t e;
     const void *src = s.dev.mom[p->parity];
     switch (p->d.storage) {
@@ -789,9 +798,8 @@ ffs_status ffs_pool_get_moments(ffs_pool *p, int slot, float *moments)
         break;
     }
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(moments, stage, sizeof(float) * 6 * (size_t)s.ncell, cudaMemcpyDeviceToHost, p->st);
+        e = cudaMemcpyAsync(moments, stage, bytes, cudaMemcpyDeviceToHost, p->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->st);
-    cudaFree(stage);
     if (e != cudaSuccess) return fail(FFS_ERR_CUDA, std::string("get_moments: ") + cudaGetErrorString(e));
     return FFS_OK;
 }
