@@ -257,40 +257,40 @@ __device__ __forceinline__ void decode_moments(float *m, const Codec &c)
 // The dither is a hash of the cell index and of the bits of the cell's new
 // density, so a cell's encoding depends only on what it stores (every kernel
 // that writes a cell gives the same bits) and changes from step to step.
-// lowbias32 (C. Wellons, "Prospecting for Hash Functions", 2018): an integer
-// mixing function with good avalanche.
+// Two multiplicative rounds with a fold between them, with the multipliers of
+// lowbias32 (C. Wellons, "Prospecting for Hash Functions", 2018): the velocity
+// takes bits 0..12, 10..22 and 16..28, whose most significant ones depend on
+// most bits of the input.
 __device__ __forceinline__ uint32_t mix32(uint32_t x)
 {
-    x ^= x >> 16;
     x *= 0x7feb352du;
     x ^= x >> 15;
-    x *= 0x846ca68bu;
-    x ^= x >> 16;
-    return x;
+    return x * 0x846ca68bu;
 }
+constexpr uint32_t kGolden = 0x9e3779b9u;
 __device__ __forceinline__ uint32_t vel_dither(size_t idx, float rho)
 {
-    return mix32((uint32_t)idx * 0x9e3779b9u ^ (uint32_t)((uint64_t)idx >> 32) ^ __float_as_uint(rho));
+    return mix32((uint32_t)idx * kGolden ^ (uint32_t)((uint64_t)idx >> 32) ^ __float_as_uint(rho));
 }
-// v rounded to binary16 stochastically with 10 random bits r: adding r << 3
-// to the magnitude bits of the float and truncating the 13 bits binary16
-// does not keep rounds up with probability (dropped bits) / 2^13, to within
-// 2^-10 of an ulp; values below binary16's normal range (2^-14) or at its
-// top round to nearest.  `back` receives the value the result represents:
-// in range, the truncated float itself (it has binary16's 11 significant
-// bits, so the conversion is exact), which saves converting back.  The add
-// goes to the whole float: below the top of the range the magnitude cannot
-// carry into the sign bit.
+// Two floats rounded to binary16 stochastically (lo in the low half), in one
+// conversion instruction: bits 0..12 of `r` decide the low value, bits 16..28
+// the high one, and a value rounds up in magnitude with probability (dropped
+// bits) / 2^13.  (The integer sequence this replaces, add 10 random bits and
+// truncate with the ends of binary16's range handled apart, took about seven
+// instructions per velocity.)
+__device__ __forceinline__ uint32_t half2_sr(float lo, float hi, uint32_t r)
+{
+    uint32_t d;
+    asm("cvt.rs.f16x2.f32 %0, %1, %2, %3;" : "=r"(d) : "f"(hi), "f"(lo), "r"(r));
+    return d;
+}
+// v rounded with bits 0..12 of r; `back` receives the value the result
+// represents.
 __device__ __forceinline__ __half half_sr(float v, uint32_t r, float &back)
 {
-    const uint32_t b = __float_as_uint(v), mag = b & 0x7fffffffu;
-    if (mag < 0x38800000u || mag >= 0x47000000u) {
-        const __half h = __float2half_rn(v);
-        back = __half2float(h);
-        return h;
-    }
-    back = __uint_as_float((b + (r << 3)) & ~0x1fffu);
-    return __float2half_rn(back);
+    const __half h = __ushort_as_half((unsigned short)half2_sr(v, 0.0f, r & 0x1fffu));
+    back = __half2float(h);
+    return h;
 }
 template <typename T> __device__ __forceinline__ T to_vel_sr(float v, uint32_t r, float &back);
 template <> __device__ __forceinline__ float to_vel_sr<float>(float v, uint32_t, float &back)
@@ -306,6 +306,10 @@ template <> __device__ __forceinline__ __nv_bfloat16 to_vel_sr<__nv_bfloat16>(fl
 {
     return __ushort_as_bfloat16(__half_as_ushort(half_sr(v, r, back)));
 }
+// Shift that takes velocity component a's 13 bits out of the cell's hash: x
+// takes bits 0..12, y bits 16..28, z bits 10..22 (its most significant bits
+// are y's least significant ones).
+__host__ __device__ constexpr int dither_shift(int a) { return a == 0 ? 0 : a == 1 ? 16 : 10; }
 
 // The stored form of moment vector m of cell idx: FP32 as is; reduced
 // storage as rho - 1, u * su (stochastically rounded) and the stress
@@ -325,7 +329,7 @@ __device__ __forceinline__ void encode_values(const float *m, size_t idx, const 
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
             float back;
-            enc[1 + a] = to_vel_sr<T>(m[1 + a] * c.su, (h >> (10 * a)) & 0x3ffu, back);
+            enc[1 + a] = to_vel_sr<T>(m[1 + a] * c.su, h >> dither_shift(a), back);
             ud[a] = back * c.inv_su;
         }
 #pragma unroll

@@ -304,10 +304,17 @@ __device__ __forceinline__ void raw_moments2(const float *f, float *R)
 // pi' = (dev * (1 - omega) / rho) + equilibrium part, which avoids
 // subtracting c_s^2 from a value near c_s^2.
 // 1 / rho from the hardware approximation refined by one Newton step (within
-// an ulp of the IEEE quotient, without the division's slow-path branch)
+// an ulp of the IEEE quotient, without the division's slow-path branch and its
+// handling of subnormal densities)
+__device__ __forceinline__ float rcp_approx(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ float recip(float x)
 {
-    float r = __fdividef(1.0f, x);
+    const float r = rcp_approx(x);
     return r * fmaf(-x, r, 2.0f);
 }
 
