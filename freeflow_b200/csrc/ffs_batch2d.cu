@@ -5,7 +5,7 @@
 // active table (dense tiles, surface elements, surface vertices); an item
 // finds its episode by a binary search over at most kPoolMaxSlots prefixes.
 // The per-item bodies are the single-grid ones (dense2d_tile or the same
-// per-cell code in strips, detect_element2_warp, link_cell_update), so a pool
+// per-cell code in strips, detect_elements2_warp, link_cell_update2), so a pool
 // episode computes bit for bit what the same
 // grid computes alone through ffs_lbm_step.  The grids are persistent
 // (a fixed number of CTAs striding over a count read from device memory), so
@@ -92,11 +92,9 @@ __global__ void pool_kinematics_kernel(const PoolEpisode *eps, const PoolParams 
 }
 
 // ---------------------------------------------------------------- detect
-// One warp per element of any episode (the single-grid body,
-// detect_element2_warp); the warp finds the element's episode once.  (Giving
-// each warp a contiguous run of elements, so that the episode search runs
-// once per run, measured no faster: the time goes to the link insertions'
-// dependent atomics, not to the search.)
+// One warp per four elements of any episodes (the single-grid body,
+// detect_elements2_warp); each group of eight lanes finds its element's
+// episode.
 template <typename T>
 __global__ void __launch_bounds__(256) pool_detect_kernel(const PoolEpisode *eps, const PoolActive *act, LinkTable lt,
                                                           uint32_t *owner, int parity)
@@ -106,15 +104,18 @@ __global__ void __launch_bounds__(256) pool_detect_kernel(const PoolEpisode *eps
     if (n == 0) return;
     const uint32_t total = act->elem_prefix[n];
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t ge = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; ge < total; ge += nwarps) {
+    const uint32_t group = (threadIdx.x & 31) >> 3;
+    for (uint32_t e0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4; e0 < total; e0 += nwarps * 4) {
+        const uint32_t ge = min(e0 + group, total - 1);
         const int a = owner_of(act->elem_prefix, n, ge);
         const uint32_t s = act->slot[a];
         const PoolEpisode &e = eps[s];
         const GridArgs<T> g = episode_args<T>(e, parity);
         const SurfaceArgs sa = episode_surface(e);
         const StepScalars sc{e.cl, e.ct, e.cf};
-        detect_element2_warp<T>(g, reinterpret_cast<uint32_t *>(e.flags), lt, sa, sc,
-                                (long long)(ge - act->elem_prefix[a]), queue[threadIdx.x >> 5], e.cell_base, owner, s);
+        detect_elements2_warp<T>(g, reinterpret_cast<uint32_t *>(e.flags), lt, sa, sc,
+                                 (long long)(ge - act->elem_prefix[a]), e0 + group < total, queue[threadIdx.x >> 5],
+                                 e.cell_base, owner, s);
     }
 }
 
@@ -282,18 +283,19 @@ __global__ void __launch_bounds__(256, 4) pool_link_cells_kernel(const PoolEpiso
     const int lane = threadIdx.x & (G - 1);
     const uint32_t group = (threadIdx.x & 31) / G;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t n = *lt.count;
-    for (uint32_t w = (((blockIdx.x * blockDim.x) + threadIdx.x) >> 5) * kPerWarp; w < n; w += nwarps * kPerWarp) {
+    const LinkItems items(lt);
+    const uint32_t n = items.n;
+    for (uint32_t w = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * kPerWarp; w < n; w += nwarps * kPerWarp) {
         // two cells per warp, possibly of different episodes; a group past the
         // end of the list rides along on the first group's cell
         const bool valid = w + group < n;
-        const uint32_t slot = lt.list[valid ? w + group : w];
+        const uint32_t slot = items.slot(lt, valid ? w + group : w);
         const PoolEpisode &e = eps[owner[slot]];
         const uint32_t cell = lt.keys[slot] - 1 - e.cell_base;
         const GridArgs<T> g = episode_args<T>(e, parity);
         const SurfaceArgs sa = episode_surface(e);
         const StepScalars sc{e.cl, e.ct, e.cf};
-        link_cell_update<2, T, false>(g, lt.links, slot, cell, e.acc, sa, sc, valid);
+        link_cell_update2<T, false, G>(g, lt.links, slot, cell, e.acc, sa, sc, valid);
         if (valid && lane < Q) lt.links[(size_t)slot * Q + lane] = ~0ull;
         __syncwarp();
         if (valid && lane == 0) {
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(256) pool_finalize_kernel(const PoolEpisode *e
 {
     __shared__ double red[4][8];
     const int n = (int)act->n;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *lt.count = 0;
+    if (blockIdx.x == 0) clear_counts(lt);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int a = blockIdx.x; a < n; a += gridDim.x) {
         const PoolEpisode &e = eps[act->slot[a]];

@@ -131,12 +131,13 @@ ffs_status ensure_links(ffs_lbm *h, int64_t max_vertices, int64_t max_link_cells
         FFS_CK(cudaMemset(lt.keys, 0, sizeof(uint32_t) * want_cap));
         FFS_CK(cudaMemset(lt.links, 0xFF, sizeof(unsigned long long) * (size_t)want_cap * h->Q));
         lt.cap = want_cap;
+        lt.seg_shift = segment_shift(want_cap);
     }
     if (!lt.count) {
-        // the list count and the finished-CTA count of link_cells_kernel
-        FFS_CK(cudaMalloc(&lt.count, 2 * sizeof(uint32_t)));
-        FFS_CK(cudaMemset(lt.count, 0, 2 * sizeof(uint32_t)));
-        lt.done = lt.count + 1;
+        // the lists' counts and the finished-CTA count of link_cells_kernel
+        FFS_CK(cudaMalloc(&lt.count, (kCountWords + 1) * sizeof(uint32_t)));
+        FFS_CK(cudaMemset(lt.count, 0, (kCountWords + 1) * sizeof(uint32_t)));
+        lt.done = lt.count + kCountWords;
     }
     if ((int64_t)lt.acc_cap < max_vertices) {
         cudaFree(lt.acc);
@@ -647,19 +648,15 @@ ffs_status ffs_lbm_debug_links(ffs_lbm *h, const ffs_surface *s, uint64_t *cell_
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);
     if (h->dim == 2) FFS_CK((launch_detect_links<2, float>(args<float>(h), words, h->lt, sa, sc, st)));
     else FFS_CK((launch_detect_links<3, float>(args<float>(h), words, h->lt, sa, sc, st)));
-    uint32_t n = 0;
-    FFS_CK(cudaMemcpyAsync(&n, h->lt.count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    FFS_CK(cudaStreamSynchronize(st));
-    std::vector<uint32_t> list(n), keys(h->lt.cap);
+    std::vector<uint32_t> keys(h->lt.cap);
     std::vector<unsigned long long> links((size_t)h->lt.cap * h->Q);
-    if (n) FFS_CK(cudaMemcpyAsync(list.data(), h->lt.list, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st));
     FFS_CK(cudaMemcpyAsync(keys.data(), h->lt.keys, sizeof(uint32_t) * h->lt.cap, cudaMemcpyDeviceToHost, st));
     FFS_CK(cudaMemcpyAsync(links.data(), h->lt.links, sizeof(unsigned long long) * links.size(), cudaMemcpyDeviceToHost, st));
     FFS_CK(cudaStreamSynchronize(st));
     std::vector<std::pair<uint64_t, uint64_t>> out;
-    for (uint32_t w = 0; w < n; ++w) {
-        uint32_t slot = list[w];
-        uint64_t cell = keys[slot] - 1;
+    for (uint32_t slot = 0; slot < h->lt.cap; ++slot) {
+        if (!keys[slot]) continue;
+        const uint64_t cell = keys[slot] - 1;
         for (int l = 0; l < h->Q; ++l) {
             unsigned long long k = links[(size_t)slot * h->Q + l];
             if (k != ~0ull) out.emplace_back(cell * h->Q + l, k);
@@ -726,7 +723,7 @@ ffs_status ffs_lbm_profile_read(ffs_lbm *h, ffs_profile *out, int reset)
 // the table has twice as many slots as the supported link cells, so it is at
 // most half full, like the table ffs_lbm_step sizes for itself):
 //   keys  [kNoallocSlots]  u32, 0 = empty slot          must start at 0
-//   list  [kNoallocSlots]  u32, claimed slots            no requirement
+//   list  [kNoallocSlots]  u32, claimed slots (one segment) no requirement
 //   count, done u32 (own 256-byte line)                  must start at 0
 //   links [kNoallocSlots * Q] u64, ~0 = no link          must start at ~0
 //   acc   [kNoallocMaxVertices * DIM] i64 force sums     must start at 0

@@ -8,19 +8,33 @@ namespace fflbm {
 // Sparse link table, rebuilt every step.  A cell that owns at least one link
 // gets one open-addressing slot: keys[slot] = cell + 1 and links[slot * Q + l]
 // = the smallest (depth, element) key of direction l (~0 if none).  `list`
-// holds the occupied slots in claim order; `count` their number.  The sparse
-// kernel returns every slot it visits to the empty state, so the table is
-// clean again at the end of the step without touching unused slots.
+// holds the occupied slots in claim order, one list per segment of the table
+// (segment = slot >> seg_shift, its list at the segment's own first slot, its
+// length in count[kCountStride * segment]).  Claims in one counter serialise:
+// they took about 1 ns each, most of detection's time in a serving pool
+// (50,000 claims a substep at 256 episodes), so a table counts in kSegments of
+// them, each in a line of its own.  The sparse kernel returns every slot it
+// visits to the empty state, so the table is clean again at the end of the
+// step without touching unused slots.
+constexpr uint32_t kSegments = 64, kCountStride = 32;
+constexpr size_t kCountWords = (size_t)kSegments * kCountStride;
 struct LinkTable {
     uint32_t cap = 0;                  // power of two (0: not allocated)
+    uint32_t seg_shift = 31;           // log2(cap / kSegments), or 31: one segment
     uint32_t *keys = nullptr;          // [cap]
     unsigned long long *links = nullptr; // [cap * Q]
     uint32_t *list = nullptr;          // [cap]
-    uint32_t *count = nullptr;         // [1]
+    uint32_t *count = nullptr;         // [kCountWords], or [1] for one segment
     long long *acc = nullptr;          // [acc_cap * DIM] fixed-point force sums (2^-32 units)
     uint32_t acc_cap = 0;              // vertices
     uint32_t *done = nullptr;          // [1] CTAs of link_cells_kernel that finished (zero between steps)
 };
+inline uint32_t segment_shift(uint32_t cap)
+{
+    uint32_t s = 0;
+    while ((cap >> s) > kSegments) ++s;
+    return s;
+}
 
 // Surfaces of at most this many force components have their fixed-point
 // sums converted by the last CTA of link_cells_kernel instead of a kernel of

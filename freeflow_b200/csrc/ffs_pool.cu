@@ -453,14 +453,15 @@ ffs_status ffs_pool_create(const ffs_pool_desc *desc, ffs_pool **out)
     while (cap < (uint64_t)link_cells * 2) cap <<= 1;
     if (cap > (1ull << 30)) return bail(cudaErrorInvalidValue, "link table too large");
     p->lt.cap = (uint32_t)cap;
+    p->lt.seg_shift = segment_shift((uint32_t)cap);
     if ((e = cudaMalloc(&p->lt.keys, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link keys");
     if ((e = cudaMalloc(&p->lt.links, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "links");
     if ((e = cudaMalloc(&p->lt.list, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link list");
-    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t))) != cudaSuccess) return bail(e, "link count");
+    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t) * kCountWords)) != cudaSuccess) return bail(e, "link count");
     if ((e = cudaMalloc(&p->owner, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link owner");
     if ((e = cudaMemset(p->lt.keys, 0, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemset(p->lt.links, 0xFF, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "memset");
-    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t))) != cudaSuccess) return bail(e, "memset");
+    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t) * kCountWords)) != cudaSuccess) return bail(e, "memset");
     p->lt.acc = nullptr; // per-episode accumulators live in the arena
     p->lt.acc_cap = 0;
     for (int sh = 0; sh < kPoolNumShapes; ++sh) {
