@@ -43,7 +43,6 @@ struct ffs_lbm {
     LinkTable lt;
     float *staging = nullptr; // ncell * NM floats, allocated on first host transfer
     uint32_t *fill_bits = nullptr; // D3Q27 solid fill: one parity bit per cell, zero between calls
-    int dense_variant = -1;   // D3Q27 kernel variant chosen on the first step (tune_dense3d)
     // link detection runs on `side` while the dense pass runs on the caller's
     // stream; fork/join order them
     cudaStream_t side = nullptr;
@@ -222,7 +221,6 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
     StepScalars sc{h->cl, h->ct, h->cf};
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);
     const bool serial = h->profiling == 2;
-    if (DIM == 3 && h->dense_variant < 0) h->dense_variant = tune_dense3d<T>(g, st);
     if (surf) {
         if (h->lt.cap == 0 || (int64_t)h->lt.acc_cap < sa.nv) {
             ffs_status r = ensure_links(h, std::max<int64_t>(sa.nv, h->lt.acc_cap),
@@ -249,7 +247,7 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
     {
         StageTimer t(h, 1, st);
         if (DIM == 2) FFS_CK(launch_dense2d<T>(g, st));
-        else FFS_CK(launch_dense3d<T>(g, st, h->dense_variant));
+        else FFS_CK(launch_dense3d<T>(g, st));
     }
     if (surf) {
         if (!serial) FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
@@ -810,7 +808,7 @@ template <int DIM, typename T> ffs_status noalloc_impl(ffs_lbm *h, const ffs_sur
         FFS_CK(cudaEventRecord(h->join, h->side));
     }
     if (DIM == 2) FFS_CK(launch_dense2d<T>(g, st));
-    else FFS_CK(launch_dense3d<T>(g, st, h->dense_variant < 0 ? 0 : h->dense_variant));
+    else FFS_CK(launch_dense3d<T>(g, st));
     if (surf) {
         FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
         const bool fold = (long long)sa.nv * DIM <= kFoldForcesMax;

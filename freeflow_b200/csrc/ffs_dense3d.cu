@@ -8,10 +8,11 @@
 // then pulls them back out of shared memory.  Here a CTA owns a 32 x 8 column
 // of cells and marches up z through a chunk of planes:
 //
-//   * each plane is reconstructed once for its 34 x 10 xy halo: every thread
-//     reconstructs its own cell, and the first 84 threads one cell of the
-//     ring around the tile as well (only the 9 populations it feeds into the
-//     tile, one kind of ring cell per warp);
+//   * each plane is reconstructed once for its 34 x 10 xy halo: eight tile
+//     warps reconstruct the tile's own cells; of the 84 cells around it only
+//     the 9 populations that point into the tile are evaluated, in FP32 by two
+//     ring warps while the tile warps still pull the plane before, in 16-bit
+//     storage by the first 84 tile threads (kRingWarps);
 //   * the populations of plane p go to one of two shared-memory buffers
 //     (2 x 27 x 340 floats) and are consumed as soon as they exist: the
 //     c_z = -1 slice completes the raw moments of the cell below (plane p-1),
@@ -39,37 +40,20 @@
 #include "ffs_dense2d.cuh"
 #include "ffs_dense3d.cuh"
 
-#include <cuda.h> // CUtensorMap and its encoder's types (the encoder is fetched at run time)
-
 #include <cstdlib>
 #include <map>
 #include <mutex>
-#include <type_traits>
 #include <utility>
 
 namespace fflbm {
 
 namespace {
-constexpr int kTX = D3::kTX, kTY = D3::kTY, kHX = D3::kHX, kHalo = D3::kHalo, kRing = D3::kRing;
+constexpr int kTX = D3::kTX, kTY = D3::kTY, kHX = D3::kHX, kHalo = D3::kHalo;
 constexpr int kPlane = D3::kPlaneFloats;
-
-__device__ __forceinline__ int set_of(int kx, int ky, int kz) { return (kz * 3 + ky) * 3 + kx; }
-
-// halo index (hx, hy) of ring cell r, grouped so that each warp holds one
-// kind of ring cell: r < 32 the row y0-1 (hx 1..32), r < 64 the row y0+8
-// (hx 1..32), r < 74 the column x0-1 (hy 0..9, corners included), r < 84
-// the column x0+32
-__device__ __forceinline__ int ring_cell(int r)
-{
-    if (r < 32) return r + 1;
-    if (r < 64) return (kHalo - kHX) + (r - 31);
-    if (r < 74) return (r - 64) * kHX;
-    return (r - 74) * kHX + kHX - 1;
-}
 
 // raw-moment slot: {rho, jx, jy, jz, Pxx, Pyy, Pzz, Pxy, Pyz, Pxz}
 //
-// Unweighted populations.  The single-plane kernel stores each population
+// Unweighted populations.  The kernel stores each population
 // as its Hermite sum F_i without the lattice weight and applies the weights
 // on the way into the raw moments.  The D3Q27 weights are one constant times
 // powers of four, w_i = W0 4^-n(i) with W0 = wgt3(1,1,1) = 8/27 and n(i) the
@@ -90,33 +74,10 @@ __device__ __forceinline__ void raw_from_scaled(const float *Rs, float *R)
     for (int k = 0; k < 10; ++k) R[k] = Rs[k] * (kW0 * s[k]);
 }
 
-// 9 unweighted populations of one c_z slice (clamped) -> x/y sums
+// The x/y sums of one c_z slice are
 // Y = {Y00, Y01, Y02, Y10, Y11, Y20}; the weighted sums are
-// W0 4^-|c_z| c_k Y_k with c = {1, 1/4, 1/4, 1/4, 1/16, 1/4}
-__device__ __forceinline__ void slice_sums(const float *buf, int kz, int c_own, float *Y)
-{
-    float X0[3], X1[3], X2[3];
-#pragma unroll
-    for (int ky = 0; ky < 3; ++ky) {
-        // population (kx, ky, kz) of the cell at c_own - (kx-1) - (ky-1)*kHX
-        const int crow = c_own - (ky - 1) * kHX;
-        float fm = fmaxf(buf[set_of(0, ky, kz) * kHalo + crow + 1], 0.0f);
-        float f0 = fmaxf(buf[set_of(1, ky, kz) * kHalo + crow], 0.0f);
-        float fp = fmaxf(buf[set_of(2, ky, kz) * kHalo + crow - 1], 0.0f);
-        float s = fp + fm;
-        X1[ky] = fp - fm;
-        X0[ky] = fmaf(0.25f, s, f0);
-        X2[ky] = s;
-    }
-    float s0 = X0[2] + X0[0];
-    Y[0] = fmaf(0.25f, s0, X0[1]);
-    Y[1] = X0[2] - X0[0];
-    Y[2] = s0;
-    Y[3] = fmaf(0.25f, X1[2] + X1[0], X1[1]);
-    Y[4] = X1[2] - X1[0];
-    Y[5] = fmaf(0.25f, X2[2] + X2[0], X2[1]);
-}
-
+// W0 4^-|c_z| c_k Y_k with c = {1, 1/4, 1/4, 1/4, 1/16, 1/4}.
+//
 // add the slice with c_z = CZ to the scaled sums R''
 template <int CZ> __device__ __forceinline__ void slice_add(float *R, const float *Y)
 {
@@ -134,25 +95,20 @@ __device__ __forceinline__ void slice_init_plus(float *R, const float *Y)
     R[3] = Y[0]; R[6] = Y[0]; R[8] = Y[1]; R[9] = Y[3];
 }
 
-// Paired layout (variant 2).  For each (c_x, c_y) set and halo cell,
+// Paired layout.  For each (c_x, c_y) set and halo cell,
 // the c_z = -1 and +1 populations sit side by side as one float2 (a plane of
 // 9 x kHalo float2), and the c_z = 0 population in a plane of floats after
 // it: the cells of a tile pull the three from the same neighbour, so one
 // 64-bit and one 32-bit load replace three, the reconstruction stores them
 // the same way, and the c_z = -1 / +1 pair is one 64-bit register pair for
-// the packed f32x2 arithmetic below.  The plane has the size of the scalar
-// layout's.  Per element, every operation is the scalar layout's, in the
-// same order: all variants give identical bits.
+// the packed f32x2 arithmetic below.  (One float plane per population took
+// 7 % more time on 384 x 192 x 192.)
 constexpr int kPairFloats = 9 * kHalo * 2;  // the float2 plane; the c_z = 0 plane follows
 // float index of population (kx, ky, kz) (k = c + 1) of halo cell c
-template <bool PAIRED> __device__ __forceinline__ int pop_index(int kx, int ky, int kz, int c)
+__device__ __forceinline__ int pop_index(int kx, int ky, int kz, int c)
 {
-    if constexpr (PAIRED) {
-        const int s9 = (kx + 3 * ky) * kHalo + c;
-        return kz == 1 ? kPairFloats + s9 : 2 * s9 + (kz == 2);
-    } else {
-        return set_of(kx, ky, kz) * kHalo + c;
-    }
+    const int s9 = (kx + 3 * ky) * kHalo + c;
+    return kz == 1 ? kPairFloats + s9 : 2 * s9 + (kz == 2);
 }
 __device__ __forceinline__ void store_pair(float *buf, int s9, f2 p, float mid)
 {
@@ -338,7 +294,6 @@ __device__ __forceinline__ void add_basis_scaled(float *R, int cx, int cy, int c
 // R'' += basis(c_i) w_i max(0, F_inv(i)(x)) (scaled as above) for every wall
 // direction i in w, with the cell's own unweighted populations read from the
 // current plane.
-template <bool PAIRED>
 __device__ __forceinline__ void add_reflected(const float *buf, int c_own, uint32_t w, float (&R)[10])
 {
 #pragma unroll
@@ -349,7 +304,7 @@ __device__ __forceinline__ void add_reflected(const float *buf, int c_own, uint3
             for (int kx = 0; kx < 3; ++kx) {
                 const int i = dir_index<3>(kx, ky, kz);
                 if (i == 0) continue;
-                float f = fmaxf(buf[pop_index<PAIRED>(2 - kx, 2 - ky, 2 - kz, c_own)], 0.0f);
+                float f = fmaxf(buf[pop_index(2 - kx, 2 - ky, 2 - kz, c_own)], 0.0f);
                 f = (w & (1u << i)) ? f : 0.0f;
                 add_basis_scaled(R, kx - 1, ky - 1, kz - 1, f);
             }
@@ -360,7 +315,6 @@ __device__ __forceinline__ void add_reflected(const float *buf, int c_own, uint3
 // face the halo cell holds real populations, but the wrapped test found a
 // wall, so the step takes the cell's reflected population instead
 // (add_reflected).
-template <bool PAIRED>
 __device__ __forceinline__ void wall_fix_part(const float *buf, int c_own, uint32_t w, int kz_sel, float (&R)[10])
 {
     while (w) {
@@ -369,7 +323,7 @@ __device__ __forceinline__ void wall_fix_part(const float *buf, int c_own, uint3
         int cx, cy, cz;
         dir_vec<3>(i, cx, cy, cz);
         if (cz + 1 == kz_sel) {
-            const float pulled = fmaxf(buf[pop_index<PAIRED>(cx + 1, cy + 1, cz + 1, c_own - cx - cy * kHX)], 0.0f);
+            const float pulled = fmaxf(buf[pop_index(cx + 1, cy + 1, cz + 1, c_own - cx - cy * kHX)], 0.0f);
             add_basis_scaled(R, cx, cy, cz, -pulled);
         }
     }
@@ -384,82 +338,30 @@ template <typename T> struct MomentPlanes {
     T *dst[10];
 };
 
-// ------------------------------------------------ staged moments (variant 3)
-// The moments of each halo plane come into shared memory by one TMA tiled
-// copy (cp.async.bulk.tensor, no multicast) two planes ahead, into one of two
-// stages, each with an mbarrier that the copy's bytes complete.  The box is
-// 4D (x, y, z, moment) over the SoA moment planes: kBX cells wide from
-// x0 - kAlign (a 16-byte boundary, as the tiled copy requires), the 10 rows
-// y0 - 1 .. y0 + 8, one plane, all 10 moments.  Cells outside the grid in x
-// or y arrive as zeros; the halo cells that lie there take the reference's
-// wrapped or clamped source with plain loads instead (halo_index).
-template <typename T> struct Stage {
-    static constexpr int kAlign = 16 / (int)sizeof(T);   // elements per 16 bytes
-    static constexpr int kOff = kAlign - 1;              // box x of halo x 0
-    static constexpr int kBX = kHX + 2 * kAlign - 2;     // 40 (FP32) or 48 (16-bit): covers halo x 0..33
-    static constexpr int kElems = kBX * D3::kHY * 10;
-    static constexpr uint32_t kBytes = (uint32_t)(kElems * sizeof(T));
-    static_assert(kBX * sizeof(T) % 16 == 0, "the box's inner extent must be a multiple of 16 bytes");
-    static_assert(kBytes % 128 == 0, "stages start on 128-byte boundaries");
-    // shared-memory layout after the two population planes
-    static constexpr size_t kBase = (D3::kSmemBytes + 127) / 128 * 128;
-    static constexpr size_t kBars = kBase + 2 * (size_t)kBytes;
-    static constexpr size_t kSmem = kBars + 2 * sizeof(uint64_t);
-};
-
-__device__ __forceinline__ uint32_t smem_u32(const void *ptr) { return (uint32_t)__cvta_generic_to_shared(ptr); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(smem_u32(bar)), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-// generic-proxy accesses of shared memory before async-proxy (TMA) ones
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2,
-                                            int c3)
-{
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
-// polls of a stage's barrier before the kernel gives up on it (status bit
-// kStatusStageTimeout; each poll may itself wait a little in hardware)
-constexpr uint32_t kStageWaitPolls = 1u << 22;
 } // namespace
 
-// MINB = CTAs per SM the register budget is cut for; launch_dense3d times the
-// variants on the grid and keeps the faster (tune_dense3d).
+// Whether the 84 halo cells around the tile have two warps of their own.  They
+// write plane p's halo populations while the tile warps still pull plane p - 1
+// from the other buffer, so the ring (a third of a cell's reconstruction per
+// tile cell) is off the tile's path between two barriers, and only they hold
+// and load ring moments; with the ring on three of the tile's own warps the
+// others wait for those at every barrier.  In FP32 that takes 128^3 from 78 to
+// 69 us and 384 x 192 x 192 from 0.53 to 0.50 ms a step.  In 16-bit storage a
+// cell's decoding makes the ring warp with two rows the slowest of the CTA: no
+// gain on 384 x 192 x 192 and 96 against 86 us on 189 x 93 x 101 (with three
+// ring warps only 80 registers are left a thread, and the pass spills), so
+// there the first 84 tile threads take a ring cell each.
+template <typename T> constexpr bool kRingWarps = !StorageTraits<T>::kEncoded;
+template <typename T> constexpr int kThreads3 = D3::kTile + (kRingWarps<T> ? 64 : 0);
+
+// One CTA: 8 warps own the 32 x 8 tile's columns, and the ring warps, where
+// there are any, the 84 halo cells around it.
 // IDX32: every moment, flag and mask index (k * ncell + cell) fits in 32
 // bits, as it does for grids of up to 429 M cells; each access then takes one
-// 32-bit index and one widening multiply-add instead of 64-bit arithmetic,
-// which saves registers (112 against 122) and about 5 % of the pass.
-// PAIRED: the paired shared-memory layout with packed c_z = -1 / +1
-// arithmetic (variant 2); otherwise one float plane per population
-// (variants 0 and 1).
-// STAGE: the halo planes' moments are staged in shared memory by TMA copies
-// through `tmap` (variant 3; IDX32 and PAIRED only); otherwise each thread
-// loads its halo cells' moments one plane ahead into registers.
-template <typename T, int MINB, bool IDX32, bool PAIRED, bool STAGE>
-__global__ void __launch_bounds__(D3::kThreads, MINB)
-    dense3d_kernel(GridArgs<T> g, const MomentPlanes<T> mp, int zchunk, const __grid_constant__ CUtensorMap tmap)
+// 32-bit index and one widening multiply-add instead of 64-bit arithmetic.
+template <typename T, bool IDX32>
+__global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g, const MomentPlanes<T> mp, int zchunk)
 {
-    static_assert(!STAGE || (IDX32 && PAIRED), "staging is built for the paired 32-bit-index kernel");
     extern __shared__ __align__(128) float smem[];
     const int tid = threadIdx.x;
     const int x0 = blockIdx.x * kTX, y0 = blockIdx.y * kTY;
@@ -467,19 +369,108 @@ __global__ void __launch_bounds__(D3::kThreads, MINB)
     const int ze = min(zb + zchunk, g.nz);
     const long long nxy = (long long)g.nx * g.ny;
     const bool wx = g.periodic & 1, wy = g.periodic & 2, wz = g.periodic & 4;
-
-    const int tx = tid % kTX, ty = tid / kTX;
-    const int x = x0 + tx, y = y0 + ty;
-    const bool inside = x < g.nx && y < g.ny;
-    const int c_own = (ty + 1) * kHX + (tx + 1);
-    // partner cell of the reconstruction pair
-    const bool has_ring = tid < kRing;
-    const int c_ring = has_ring ? ring_cell(tid) : c_own;
     auto planar = [&](int c) {
         int hx = c % kHX, hy = c / kHX;
         return (uint32_t)(halo_index(y0 + hy - 1, g.ny, wy) * g.nx + halo_index(x0 + hx - 1, g.nx, wx));
     };
-    const uint32_t off_own = planar(c_own), off_ring = planar(c_ring);
+    // halo cells beyond a high face keep their real populations even when
+    // they are walls (x and y per thread, z per plane)
+    auto beyond_hi = [&](int c) {
+        const int hx = x0 + c % kHX - 1, hy = y0 + c / kHX - 1;
+        return (!wx && hx >= g.nx) || (!wy && hy >= g.ny);
+    };
+    // stored moments and node type of one halo cell in plane z
+    auto load_cell = [&](int z, uint32_t off, T (&m)[10], uint32_t &h) {
+        if constexpr (IDX32) {
+            const uint32_t i = (uint32_t)halo_index(z, g.nz, wz) * (uint32_t)nxy + off;
+#pragma unroll
+            for (int k = 0; k < 10; ++k) m[k] = mp.src[k][i];
+            h = g.flags[i] & kTypeMask;
+        } else {
+            const size_t i = (size_t)halo_index(z, g.nz, wz) * nxy + off;
+#pragma unroll
+            for (int k = 0; k < 10; ++k) m[k] = g.src[(size_t)k * g.ncell + i];
+            h = g.flags[i] & kTypeMask;
+        }
+    };
+    auto coefficients = [&](const T *raw) {
+        float m[10];
+#pragma unroll
+        for (int k = 0; k < 10; ++k) m[k] = from_storage<3, T>(k, raw[k]);
+        decode_moments<3, T>(m, g.codec);
+        Coef3V<float> cf;
+        cf.make(m);
+        return cf;
+    };
+
+    if (kRingWarps<T> && tid >= D3::kTile) {
+        // ---- ring warps.  A ring cell feeds the tile only the 9 populations
+        // that point into it: the first warp evaluates c_y = +1 of the row
+        // below and c_y = -1 of the row above, the second c_x = +-1 of the
+        // columns (10 cells each).  No other slot of a ring cell is ever read.
+        const int lane = tid & 31;
+        auto zero_slot = [&](uint32_t h, bool hi, int p) { return is_bounce_back<3>(h) && !(hi || (!wz && p >= g.nz)); };
+        const f2 z2 = f2make(0.0f, 0.0f);
+        if (tid < D3::kTile + 32) {
+            const int cb = lane + 1, ca = kHalo - kHX + lane + 1;
+            const uint32_t ob = planar(cb), oa = planar(ca);
+            const bool hib = beyond_hi(cb), hia = beyond_hi(ca);
+            T rb[10], ra[10];
+            uint32_t hb = 0, ha = 0;
+            load_cell(zb - 1, ob, rb, hb);
+            load_cell(zb - 1, oa, ra, ha);
+            for (int p = zb - 1; p <= ze; ++p) {
+                float *buf = smem + (p & 1) * kPlane;
+                if (zero_slot(hb, hib, p)) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) store_pair(buf, (k + 6) * kHalo + cb, z2, 0.0f);
+                } else {
+                    store_row_paired<2>(coefficients(rb), buf, cb);
+                }
+                if (p < ze) load_cell(p + 1, ob, rb, hb);
+                if (zero_slot(ha, hia, p)) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) store_pair(buf, k * kHalo + ca, z2, 0.0f);
+                } else {
+                    store_row_paired<0>(coefficients(ra), buf, ca);
+                }
+                if (p < ze) load_cell(p + 1, oa, ra, ha);
+                __syncthreads(); // plane p is in buf; the tile has left the other buffer
+            }
+        } else {
+            const bool has = lane < 2 * D3::kHY, left = lane < D3::kHY;
+            const int c = left ? lane * kHX : ((has ? lane : 2 * D3::kHY - 1) - D3::kHY) * kHX + kHX - 1;
+            const uint32_t off = planar(c);
+            const bool hi = beyond_hi(c);
+            const float sx = left ? 1.0f : -1.0f; // c_x of the fed populations
+            const int kx = left ? 2 : 0;          // and its index
+            T raw[10];
+            uint32_t h = 0;
+            load_cell(zb - 1, off, raw, h);
+            for (int p = zb - 1; p <= ze; ++p) {
+                float *buf = smem + (p & 1) * kPlane;
+                if (has) {
+                    if (zero_slot(h, hi, p)) {
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) store_pair(buf, (kx + 3 * k) * kHalo + c, z2, 0.0f);
+                    } else {
+                        store_col_paired(coefficients(raw), sx, kx, buf, c);
+                    }
+                }
+                if (p < ze) load_cell(p + 1, off, raw, h);
+                __syncthreads();
+            }
+        }
+        return;
+    }
+
+    // ---- tile warps
+    const int tx = tid % kTX, ty = tid / kTX;
+    const int x = x0 + tx, y = y0 + ty;
+    const bool inside = x < g.nx && y < g.ny;
+    const int c_own = (ty + 1) * kHX + (tx + 1);
+    const uint32_t off_own = planar(c_own);
+    const bool own_hi = beyond_hi(c_own);
     const uint32_t col = inside ? (uint32_t)(y * g.nx + x) : 0u;
     // directions whose pull crosses the high x or y face of a non-periodic
     // axis (only there can the halo cell and the wrapped test differ)
@@ -501,184 +492,61 @@ __global__ void __launch_bounds__(D3::kThreads, MINB)
             if (cz == -1) oor_zhi |= 1u << i;
         }
     }
-    // halo cells beyond a high face keep their real populations even when
-    // they are walls (x and y per thread, z per plane)
-    auto beyond_hi = [&](int c) {
-        const int hx = x0 + c % kHX - 1, hy = y0 + c / kHX - 1;
-        return (!wx && hx >= g.nx) || (!wy && hy >= g.ny);
-    };
-    const bool own_hi = beyond_hi(c_own), ring_hi = beyond_hi(c_ring);
-
-    // stored moments of the two halo cells, converted when they are
-    // reconstructed (so that only the ring warps convert the ring cell's;
-    // the loads themselves stay predicated in every warp, which overlaps them
-    // with the own-cell loads: a warp-uniform branch around the ring loads
-    // measured 9 % slower on 384 x 192 x 192)
-    T mA[10], mB[10];
-    uint32_t hA = 0, hB = 0; // node types of the two halo cells (bounce-back cells get zero slots)
-    auto load_plane = [&](int z) {
-        if constexpr (STAGE) {
-            // moments arrive by the staged copies; the halo cells' node types
-            // still come one plane ahead
-            const uint32_t zo = (uint32_t)halo_index(z, g.nz, wz) * (uint32_t)nxy;
-            hA = g.flags[zo + off_own] & kTypeMask;
-            if (has_ring) hB = g.flags[zo + off_ring] & kTypeMask;
-        } else if constexpr (IDX32) {
-            const uint32_t zo = (uint32_t)halo_index(z, g.nz, wz) * (uint32_t)nxy;
-            const uint32_t io = zo + off_own, ir = zo + off_ring;
-#pragma unroll
-            for (int k = 0; k < 10; ++k) {
-                mA[k] = mp.src[k][io];
-                if (has_ring) mB[k] = mp.src[k][ir];
-            }
-            hA = g.flags[io] & kTypeMask;
-            if (has_ring) hB = g.flags[ir] & kTypeMask;
+    // the column's halo cell of the next plane, converted when it is reconstructed
+    T raw[10];
+    uint32_t h = 0;
+    // without ring warps: the thread's ring cell (the row below: warp 0, the
+    // row above: warp 1, the columns: warp 2, so each warp runs one path)
+    const bool has_ring = !kRingWarps<T> && tid < D3::kRing;
+    const bool left = tid < 64 + D3::kHY;
+    int c_ring = c_own;
+    if (has_ring)
+        c_ring = tid < 32   ? tid + 1
+                 : tid < 64 ? kHalo - kHX + tid - 31
+                 : left     ? (tid - 64) * kHX
+                            : (tid - 64 - D3::kHY) * kHX + kHX - 1;
+    const uint32_t off_ring = kRingWarps<T> ? 0u : planar(c_ring);
+    const bool ring_hi = !kRingWarps<T> && beyond_hi(c_ring);
+    T rawr[10];
+    uint32_t hr = 0;
+    auto load_own = [&](int z) {
+        if constexpr (kRingWarps<T>) {
+            load_cell(z, off_own, raw, h);
         } else {
-            const size_t zo = (size_t)halo_index(z, g.nz, wz) * nxy;
-            const T *base = g.src + zo;
+            // the ring loads are predicated one by one, which overlaps them with
+            // the own-cell loads: a branch around them measured 9 % slower on
+            // 384 x 192 x 192
+            const size_t zo = IDX32 ? (size_t)0 : (size_t)halo_index(z, g.nz, wz) * nxy;
+            const uint32_t z32 = IDX32 ? (uint32_t)halo_index(z, g.nz, wz) * (uint32_t)nxy : 0u;
+            const uint32_t io = z32 + off_own, ir = z32 + off_ring;
 #pragma unroll
             for (int k = 0; k < 10; ++k) {
-                mA[k] = base[(size_t)k * g.ncell + off_own];
-                if (has_ring) mB[k] = base[(size_t)k * g.ncell + off_ring];
+                const T *plane = IDX32 ? mp.src[k] : g.src + (size_t)k * g.ncell + zo;
+                raw[k] = plane[io];
+                if (has_ring) rawr[k] = plane[ir];
             }
-            hA = g.flags[zo + off_own] & kTypeMask;
-            if (has_ring) hB = g.flags[zo + off_ring] & kTypeMask;
+            h = g.flags[zo + io] & kTypeMask;
+            if (has_ring) hr = g.flags[zo + ir] & kTypeMask;
         }
+    };
+    auto store_ring = [&](float *buf, int p) {
+        const int kx = left ? 2 : 0;
+        const f2 z2 = f2make(0.0f, 0.0f);
+        if (is_bounce_back<3>(hr) && !(ring_hi || (!wz && p >= g.nz))) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                store_pair(buf, (tid < 32 ? k + 6 : tid < 64 ? k : kx + 3 * k) * kHalo + c_ring, z2, 0.0f);
+            return;
+        }
+        const Coef3V<float> cf = coefficients(rawr);
+        if (tid < 32) store_row_paired<2>(cf, buf, c_ring);
+        else if (tid < 64) store_row_paired<0>(cf, buf, c_ring);
+        else store_col_paired(cf, left ? 1.0f : -1.0f, kx, buf, c_ring);
     };
     // index of the column's cell in plane z (32 or 64-bit, as above)
     auto cell_at = [&](int z) {
         if constexpr (IDX32) return (size_t)((uint32_t)z * (uint32_t)nxy + col);
         else return (size_t)z * nxy + col;
-    };
-    auto recon_cell = [&](float *buf, const T *raw, bool zero, int c) {
-        if (zero) {
-            if constexpr (PAIRED) {
-#pragma unroll
-                for (int j = 0; j < 9; ++j) store_pair(buf, j * kHalo + c, f2make(0.0f, 0.0f), 0.0f);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 27; ++j) buf[j * kHalo + c] = 0.0f;
-            }
-            return;
-        }
-        float m[10];
-#pragma unroll
-        for (int k = 0; k < 10; ++k) m[k] = from_storage<3, T>(k, raw[k]);
-        decode_moments<3, T>(m, g.codec);
-        Coef3V<float> cf;
-        cf.make(m);
-        if constexpr (PAIRED) store_populations_paired(cf, buf, c);
-        else cf.populations_each<false>([&](int kz, int ky, int kx, float v) { buf[set_of(kx, ky, kz) * kHalo + c] = v; });
-    };
-    // A ring cell feeds the tile only the 9 populations that point into it:
-    // c_y = +1 from the row below (warp 0), c_y = -1 from the row above
-    // (warp 1), c_x = +-1 from the columns (warp 2).  Each warp runs one
-    // uniform path that evaluates just those; no other slot of a ring cell is
-    // ever read.
-    const int ring_kind = tid < 32 ? 0 : tid < 64 ? 1 : 2;
-    const float ring_sx = tid < 74 ? 1.0f : -1.0f;                 // columns: c_x of the fed populations
-    const int ring_kx = tid < 74 ? 2 : 0;                          // their kx = c_x + 1
-    const int ring_kxo = ring_kx * kHalo;                          // and its plane offset
-    auto recon_ring = [&](float *buf, const T *raw, bool zero) {
-        const int c = c_ring;
-        if (zero) {
-            if constexpr (PAIRED) {
-                const f2 z2 = f2make(0.0f, 0.0f);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    if (ring_kind == 0) store_pair(buf, (k + 6) * kHalo + c, z2, 0.0f);
-                    else if (ring_kind == 1) store_pair(buf, k * kHalo + c, z2, 0.0f);
-                    else store_pair(buf, (ring_kx + 3 * k) * kHalo + c, z2, 0.0f);
-                }
-            } else {
-#pragma unroll
-                for (int kz = 0; kz < 3; ++kz)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        if (ring_kind == 0) buf[set_of(k, 2, kz) * kHalo + c] = 0.0f;
-                        else if (ring_kind == 1) buf[set_of(k, 0, kz) * kHalo + c] = 0.0f;
-                        else buf[set_of(0, k, kz) * kHalo + ring_kxo + c] = 0.0f;
-                    }
-            }
-            return;
-        }
-        float m[10];
-#pragma unroll
-        for (int k = 0; k < 10; ++k) m[k] = from_storage<3, T>(k, raw[k]);
-        decode_moments<3, T>(m, g.codec);
-        Coef3V<float> cf;
-        cf.make(m);
-        if constexpr (PAIRED) {
-            if (ring_kind == 0) store_row_paired<2>(cf, buf, c);
-            else if (ring_kind == 1) store_row_paired<0>(cf, buf, c);
-            else store_col_paired(cf, ring_sx, ring_kx, buf, c);
-            return;
-        }
-        if (ring_kind == 0)
-            cf.populations_row<2>([&](int kz, int kx, float v) { buf[set_of(kx, 2, kz) * kHalo + c] = v; });
-        else if (ring_kind == 1)
-            cf.populations_row<0>([&](int kz, int kx, float v) { buf[set_of(kx, 0, kz) * kHalo + c] = v; });
-        else
-            cf.populations_col(ring_sx, [&](int kz, int ky, float v) { buf[set_of(0, ky, kz) * kHalo + ring_kxo + c] = v; });
-    };
-    // plane p's halo cells; bounce-back cells get zero slots unless they lie
-    // beyond a high face
-    // Staging (STAGE): stage s of plane q is (q - zb + 1) & 1, its use
-    // count (q - zb + 1) >> 1 the barrier phase to wait for.
-    using SG = Stage<T>;
-    T *stage_mem = reinterpret_cast<T *>(reinterpret_cast<char *>(smem) + SG::kBase);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(smem) + SG::kBars);
-    bool stage_ok = true;
-    // halo cells outside the grid in x or y come by plain loads
-    auto outside_xy = [&](int c) {
-        const int hx = x0 + c % kHX - 1, hy = y0 + c / kHX - 1;
-        return hx < 0 || hx >= g.nx || hy < 0 || hy >= g.ny;
-    };
-    const bool own_direct = outside_xy(c_own), ring_direct = outside_xy(c_ring);
-    auto issue_plane = [&](int q) { // thread 0 only
-        const int sidx = (q - zb + 1) & 1;
-        mbar_expect_tx(&bars[sidx], SG::kBytes);
-        tma_load_4d(stage_mem + (size_t)sidx * SG::kElems, &tmap, &bars[sidx], x0 - SG::kAlign, y0 - 1,
-                    halo_index(q, g.nz, wz), 0);
-    };
-    auto fetch = [&](int q, int c, bool direct, uint32_t off, T (&raw)[10]) {
-        if (direct) {
-            const uint32_t io = (uint32_t)halo_index(q, g.nz, wz) * (uint32_t)nxy + off;
-#pragma unroll
-            for (int k = 0; k < 10; ++k) raw[k] = mp.src[k][io];
-        } else {
-            const T *st = stage_mem + (size_t)((q - zb + 1) & 1) * SG::kElems;
-            const int e = (c / kHX) * SG::kBX + c % kHX + SG::kOff;
-#pragma unroll
-            for (int k = 0; k < 10; ++k) raw[k] = st[k * (D3::kHY * SG::kBX) + e];
-        }
-    };
-    auto recon_plane = [&](float *buf, int p) {
-        const bool zhi = !wz && p >= g.nz;
-        if constexpr (STAGE) {
-            const int sidx = (p - zb + 1) & 1;
-            const uint32_t parity = (uint32_t)((p - zb + 1) >> 1) & 1u;
-            if (stage_ok) {
-                uint32_t polls = 0;
-                while (!mbar_try_wait(&bars[sidx], parity)) {
-                    if (++polls >= kStageWaitPolls) {
-                        atomicOr(g.status, kStatusStageTimeout);
-                        stage_ok = false;
-                        break;
-                    }
-                }
-            }
-            T raw[10];
-            fetch(p, c_own, own_direct, off_own, raw);
-            recon_cell(buf, raw, is_bounce_back<3>(hA) && !(own_hi || zhi), c_own);
-            if (has_ring) {
-                fetch(p, c_ring, ring_direct, off_ring, raw);
-                recon_ring(buf, raw, is_bounce_back<3>(hB) && !(ring_hi || zhi));
-            }
-        } else {
-            recon_cell(buf, mA, is_bounce_back<3>(hA) && !(own_hi || zhi), c_own);
-            if (has_ring) recon_ring(buf, mB, is_bounce_back<3>(hB) && !(ring_hi || zhi));
-        }
     };
     auto flag_at = [&](int z) -> uint32_t {
         return (inside && z >= zb && z < ze) ? (uint32_t)g.flags[cell_at(z)] : 0u;
@@ -697,8 +565,17 @@ __global__ void __launch_bounds__(D3::kThreads, MINB)
     // Rn receives the new c_z = +1 slice (the cell at z = p+1)
     auto plane = [&](int p, float (&Rp)[10], float (&Rc)[10]) {
         float *buf = smem + (p & 1) * kPlane;
-        recon_plane(buf, p);
-        if (p < ze) load_plane(p + 1);
+        // bounce-back cells get zero slots unless they lie beyond a high face
+        if (is_bounce_back<3>(h) && !(own_hi || (!wz && p >= g.nz))) {
+#pragma unroll
+            for (int j = 0; j < 9; ++j) store_pair(buf, j * kHalo + c_own, f2make(0.0f, 0.0f), 0.0f);
+        } else {
+            store_populations_paired(coefficients(raw), buf, c_own);
+        }
+        if constexpr (!kRingWarps<T>) {
+            if (has_ring) store_ring(buf, p);
+        }
+        if (p < ze) load_own(p + 1);
         const uint32_t fnn = flag_at(p + 2);
         // mask word (wall and outlet bits) of the cell at z = p+1; only cells
         // this pass updates use it (walls, inlets and outlets carry mask bits
@@ -706,13 +583,6 @@ __global__ void __launch_bounds__(D3::kThreads, MINB)
         const bool upd_n = is_updated(fn & kTypeMask) && !(fn & kBitLink);
         const uint32_t wn = (upd_n && (fn & (kBitNearWall | kBitOutletSrc))) ? g.wallmask[cell_at(p + 1)] : 0u;
         __syncthreads();
-        if constexpr (STAGE) {
-            // every thread has read plane p's stage: refill it with plane p + 2
-            if (tid == 0 && stage_ok && p + 2 <= ze) {
-                fence_proxy_async();
-                issue_plane(p + 2);
-            }
-        }
         if (inside) {
             constexpr uint32_t kWall = wall_bits_mask<3>();
             // the cell at z = p - 1 is complete: collide, store, feed outlets
@@ -736,82 +606,36 @@ __global__ void __launch_bounds__(D3::kThreads, MINB)
             // populations): remove the pulled value, per destination cell
             // z = p-1 (c_z = -1 slice) and z = p (c_z = 0)
             const uint32_t oor_p = oor_xy | ((p - 1 == g.nz - 1) ? oor_zhi : 0u);
-            if constexpr (PAIRED) {
-                f2 Sp[6];
-                float Sm[6], lo[6], hi[6];
-                slice_sums_paired(buf, c_own, Sp, Sm);
+            f2 Sp[6];
+            float Sm[6], lo[6], hi[6];
+            slice_sums_paired(buf, c_own, Sp, Sm);
 #pragma unroll
-                for (int k = 0; k < 6; ++k) f2split(Sp[k], lo[k], hi[k]);
-                slice_add<-1>(Rp, lo);
-                slice_add<0>(Rc, Sm);
-                if ((wc | wp) & kWall) { // near-wall cells only: one test on the common path
-                    if (wc & kWall) add_reflected<PAIRED>(buf, c_own, wc & kWall, Rc);
-                    if (wp & kWall & oor_p) wall_fix_part<PAIRED>(buf, c_own, wp & kWall & oor_p, 0, Rp);
-                    if (wc & kWall & oor_xy) wall_fix_part<PAIRED>(buf, c_own, wc & kWall & oor_xy, 1, Rc);
-                }
-                float R[10];
-                raw_from_scaled(Rp, R);
-                // Rp is free: it becomes the cell at z = p + 1
-                slice_init_plus(Rp, hi);
-                if (wn & kWall & oor_xy) wall_fix_part<PAIRED>(buf, c_own, wn & kWall & oor_xy, 2, Rp);
-                finish(R);
-            } else {
-                float S[6];
-                slice_sums(buf, 0, c_own, S);
-                slice_add<-1>(Rp, S);
-                slice_sums(buf, 1, c_own, S);
-                slice_add<0>(Rc, S);
-                if ((wc | wp) & kWall) {
-                    if (wc & kWall) add_reflected<PAIRED>(buf, c_own, wc & kWall, Rc);
-                    if (wp & kWall & oor_p) wall_fix_part<PAIRED>(buf, c_own, wp & kWall & oor_p, 0, Rp);
-                    if (wc & kWall & oor_xy) wall_fix_part<PAIRED>(buf, c_own, wc & kWall & oor_xy, 1, Rc);
-                }
-                {
-                    float R[10];
-                    raw_from_scaled(Rp, R);
-                    finish(R);
-                }
-                // Rp is free: it becomes the cell at z = p + 1
-                slice_sums(buf, 2, c_own, S);
-                slice_init_plus(Rp, S);
-                if (wn & kWall & oor_xy) wall_fix_part<PAIRED>(buf, c_own, wn & kWall & oor_xy, 2, Rp);
+            for (int k = 0; k < 6; ++k) f2split(Sp[k], lo[k], hi[k]);
+            slice_add<-1>(Rp, lo);
+            slice_add<0>(Rc, Sm);
+            if ((wc | wp) & kWall) { // near-wall cells only: one test on the common path
+                if (wc & kWall) add_reflected(buf, c_own, wc & kWall, Rc);
+                if (wp & kWall & oor_p) wall_fix_part(buf, c_own, wp & kWall & oor_p, 0, Rp);
+                if (wc & kWall & oor_xy) wall_fix_part(buf, c_own, wc & kWall & oor_xy, 1, Rc);
             }
+            float R[10];
+            raw_from_scaled(Rp, R);
+            // Rp is free: it becomes the cell at z = p + 1
+            slice_init_plus(Rp, hi);
+            if (wn & kWall & oor_xy) wall_fix_part(buf, c_own, wn & kWall & oor_xy, 2, Rp);
+            finish(R);
         }
         fp = fc; fc = fn; fn = fnn;
         wp = wc; wc = wn;
     };
 
-    if constexpr (STAGE) {
-        if (tid == 0) {
-            mbar_init(&bars[0], 1);
-            mbar_init(&bars[1], 1);
-            mbar_init_fence();
-        }
-        __syncthreads();
-        if (tid == 0) {
-            issue_plane(zb - 1);
-            issue_plane(zb);
-        }
-    }
-    load_plane(zb - 1);
+    load_own(zb - 1);
     int p = zb - 1;
     for (; p + 1 <= ze; p += 2) {
         plane(p, X, Y);     // completes X (z = p-1); X := z = p+1
         plane(p + 1, Y, X); // completes Y (z = p);   Y := z = p+2
     }
     if (p <= ze) plane(p, X, Y);
-    if constexpr (STAGE) {
-        // after a wait gave up, wait (bounded) for the copies still in flight
-        // into this CTA's shared memory before it exits
-        if (!stage_ok && tid == 0) {
-            for (int q = max(zb - 1, ze - 1); q <= ze; ++q) {
-                const int sidx = (q - zb + 1) & 1;
-                const uint32_t parity = (uint32_t)((q - zb + 1) >> 1) & 1u;
-                for (uint32_t polls = 0; polls < kStageWaitPolls && !mbar_try_wait(&bars[sidx], parity); ++polls) {
-                }
-            }
-        }
-    }
 }
 
 // CTAs of `kernel` resident on the current device at once (SMs x occupancy),
@@ -862,151 +686,36 @@ static int choose_zchunks(int tiles, int nz, int slots)
     return best;
 }
 
-// cuTensorMapEncodeTiled, fetched from the driver once (the library links
-// only the runtime).  Null when the driver does not offer it.
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiled tensor_map_encoder()
+template <typename T, bool IDX32> static cudaError_t launch_as(const GridArgs<T> &g, cudaStream_t s)
 {
-    static const EncodeTiled fn = []() -> EncodeTiled {
-        void *ptr = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &ptr, 12000, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<EncodeTiled>(ptr);
-    }();
-    return fn;
-}
-
-// The staged copies' tensor map over the source moments: 4D (x, y, z,
-// moment), box (kBX, 10, 1, 10), zeros outside the grid.  False when the
-// grid cannot be staged: a row of moments must be a multiple of 16 bytes
-// (nx a multiple of 4 in FP32, of 8 in 16-bit storage), indices must fit in
-// 32 bits, or the encoder refuses the shape.
-template <typename T> static bool stage_map(const GridArgs<T> &g, CUtensorMap &map)
-{
-    if (((size_t)g.nx * sizeof(T)) % 16 != 0 || reinterpret_cast<uintptr_t>(g.src) % 16 != 0) return false;
-    if (10ull * g.ncell > 0xFFFFFFFFull) return false;
-    const EncodeTiled enc = tensor_map_encoder();
-    if (!enc) return false;
-    const size_t es = sizeof(T);
-    const cuuint64_t dims[4] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz, 10};
-    const cuuint64_t strides[3] = {(cuuint64_t)g.nx * es, (cuuint64_t)g.nx * g.ny * es, (cuuint64_t)g.ncell * es};
-    const cuuint32_t box[4] = {(cuuint32_t)Stage<T>::kBX, (cuuint32_t)D3::kHY, 1, 10};
-    const cuuint32_t estride[4] = {1, 1, 1, 1};
-    const CUtensorMapDataType dt = es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
-    return enc(&map, dt, 4, const_cast<T *>(g.src), dims, strides, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <typename T, int MINB, bool IDX32, bool PAIRED, bool STAGE> struct Dense3dLaunchAs {
-    static cudaError_t run(const GridArgs<T> &g, cudaStream_t s, const CUtensorMap &map)
-    {
-        int slots = 0;
-        constexpr size_t smem = STAGE ? Stage<T>::kSmem : D3::kSmemBytes;
-        cudaError_t e = resident_slots(reinterpret_cast<const void *>(dense3d_kernel<T, MINB, IDX32, PAIRED, STAGE>),
-                                       D3::kThreads, smem, slots);
-        if (e != cudaSuccess) return e;
-        int tx = (g.nx + kTX - 1) / kTX, ty = (g.ny + kTY - 1) / kTY;
-        int nchunk = choose_zchunks(tx * ty, g.nz, slots);
-        int zchunk = (g.nz + nchunk - 1) / nchunk;
-        dim3 grid(tx, ty, (g.nz + zchunk - 1) / zchunk);
-        MomentPlanes<T> mp;
-        for (int k = 0; k < 10; ++k) {
-            mp.src[k] = g.src + (size_t)k * g.ncell;
-            mp.dst[k] = g.dst + (size_t)k * g.ncell;
-        }
-        dense3d_kernel<T, MINB, IDX32, PAIRED, STAGE><<<grid, D3::kThreads, smem, s>>>(g, mp, zchunk, map);
-        return cudaGetLastError();
+    int slots = 0;
+    const cudaError_t e =
+        resident_slots(reinterpret_cast<const void *>(dense3d_kernel<T, IDX32>), kThreads3<T>, D3::kSmemBytes, slots);
+    if (e != cudaSuccess) return e;
+    int tx = (g.nx + kTX - 1) / kTX, ty = (g.ny + kTY - 1) / kTY;
+    int nchunk = choose_zchunks(tx * ty, g.nz, slots);
+    int zchunk = (g.nz + nchunk - 1) / nchunk;
+    dim3 grid(tx, ty, (g.nz + zchunk - 1) / zchunk);
+    MomentPlanes<T> mp;
+    for (int k = 0; k < 10; ++k) {
+        mp.src[k] = g.src + (size_t)k * g.ncell;
+        mp.dst[k] = g.dst + (size_t)k * g.ncell;
     }
-};
+    dense3d_kernel<T, IDX32><<<grid, kThreads3<T>, D3::kSmemBytes, s>>>(g, mp, zchunk);
+    return cudaGetLastError();
+}
 
 // 32-bit indices whenever every moment index of the grid fits (FFS_DENSE3D_INDEX64
 // forces 64-bit indices, so that tests reach that path on small grids)
-template <typename T, int MINB, bool PAIRED> struct Dense3dLaunch {
-    static cudaError_t run(const GridArgs<T> &g, cudaStream_t s)
-    {
-        const CUtensorMap none{};
-        const char *force64 = std::getenv("FFS_DENSE3D_INDEX64");
-        if (10ull * g.ncell <= 0xFFFFFFFFull && !(force64 && force64[0] == '1'))
-            return Dense3dLaunchAs<T, MINB, true, PAIRED, false>::run(g, s, none);
-        return Dense3dLaunchAs<T, MINB, false, PAIRED, false>::run(g, s, none);
-    }
-};
-
-// Variant 3: staged moments; grids that cannot be staged run variant 2.
-template <typename T> static cudaError_t launch_staged(const GridArgs<T> &g, cudaStream_t s)
+template <typename T> cudaError_t launch_dense3d(const GridArgs<T> &g, cudaStream_t s)
 {
-    CUtensorMap map;
-    if (!stage_map(g, map)) return Dense3dLaunch<T, 2, true>::run(g, s);
-    return Dense3dLaunchAs<T, 2, true, true, true>::run(g, s, map);
+    const char *force64 = std::getenv("FFS_DENSE3D_INDEX64");
+    if (10ull * g.ncell <= 0xFFFFFFFFull && !(force64 && force64[0] == '1')) return launch_as<T, true>(g, s);
+    return launch_as<T, false>(g, s);
 }
 
-
-template <typename T> bool dense3d_has_variant(int v, const GridArgs<T> &g)
-{
-    if (v == 3) {
-        CUtensorMap map;
-        return stage_map(g, map);
-    }
-    return v >= 0 && v < kDense3dVariants;
-}
-
-template <typename T>
-cudaError_t launch_dense3d(const GridArgs<T> &g, cudaStream_t s, int variant)
-{
-    switch (variant) {
-    case 1: return Dense3dLaunch<T, 3, false>::run(g, s);
-    case 2: return Dense3dLaunch<T, 2, true>::run(g, s);
-    case 3: return launch_staged<T>(g, s);
-    default: return Dense3dLaunch<T, 2, false>::run(g, s);
-    }
-}
-
-// Times each variant on this grid (the pass only reads src and writes dst, so
-// repeating it is harmless) and returns the fastest.  Variant 2 is timed
-// first and kept unless another is at least 1 % faster: all give the same
-// bits, so the margin only keeps the choice stable, and on B200 variant 2 is
-// the fastest for FP32 and FP16 storage.
-template <typename T>
-int tune_dense3d(const GridArgs<T> &g, cudaStream_t s)
-{
-    // FFS_DENSE3D_VARIANT pins the variant (tests run every variant this way)
-    if (const char *pin = std::getenv("FFS_DENSE3D_VARIANT")) {
-        const int v = std::atoi(pin);
-        if (dense3d_has_variant<T>(v, g)) return v;
-    }
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    float best = 1e30f;
-    int best_v = -1;
-    constexpr int kOrder[kDense3dVariants] = {2, 0, 1, 3};
-    for (int v : kOrder) {
-        if (!dense3d_has_variant<T>(v, g)) continue;
-        if (launch_dense3d<T>(g, s, v) != cudaSuccess) continue; // warm-up
-        cudaEventRecord(a, s);
-        for (int r = 0; r < 5; ++r) launch_dense3d<T>(g, s, v);
-        cudaEventRecord(b, s);
-        cudaEventSynchronize(b);
-        float ms = 0.0f;
-        cudaEventElapsedTime(&ms, a, b);
-        if (best_v < 0 || ms < 0.99f * best) { best = ms; best_v = v; }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    return best_v < 0 ? 0 : best_v;
-}
-
-template cudaError_t launch_dense3d<float>(const GridArgs<float> &, cudaStream_t, int);
-template cudaError_t launch_dense3d<__half>(const GridArgs<__half> &, cudaStream_t, int);
-template cudaError_t launch_dense3d<__nv_bfloat16>(const GridArgs<__nv_bfloat16> &, cudaStream_t, int);
-template int tune_dense3d<float>(const GridArgs<float> &, cudaStream_t);
-template int tune_dense3d<__half>(const GridArgs<__half> &, cudaStream_t);
-template int tune_dense3d<__nv_bfloat16>(const GridArgs<__nv_bfloat16> &, cudaStream_t);
+template cudaError_t launch_dense3d<float>(const GridArgs<float> &, cudaStream_t);
+template cudaError_t launch_dense3d<__half>(const GridArgs<__half> &, cudaStream_t);
+template cudaError_t launch_dense3d<__nv_bfloat16>(const GridArgs<__nv_bfloat16> &, cudaStream_t);
 
 } // namespace fflbm
