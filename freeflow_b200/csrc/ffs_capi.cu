@@ -2,8 +2,9 @@
 // memory, and the per-step launch sequence.
 //
 // Per step, on the caller's stream and without host synchronisation:
-//   1. detect_links   (only with a surface)   O(surface), on a side stream,
-//                                             concurrent with 2
+//   1. detect_links   (only with a surface)   O(surface): in blocks of 2's
+//                                             launch (D2Q9), or on a side
+//                                             stream, concurrent with 2
 //   2. dense2d/dense3d                         O(grid), the bandwidth-bound pass
 //   3. link_cells     (only with a surface)   O(boundary cells), after 1 and 2
 //   4. finalize_forces(only with a surface)   O(vertices); folded into the
@@ -221,6 +222,10 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
     StepScalars sc{h->cl, h->ct, h->cf};
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);
     const bool serial = h->profiling == 2;
+    // 2D grids detect links in blocks of the dense pass's launch; stage timing
+    // keeps the stages apart
+    bool merged = false;
+    if constexpr (DIM == 2) merged = surf && !h->profiling && dense2d_detects<T>(g);
     if (surf) {
         if (h->lt.cap == 0 || (int64_t)h->lt.acc_cap < sa.nv) {
             ffs_status r = ensure_links(h, std::max<int64_t>(sa.nv, h->lt.acc_cap),
@@ -234,27 +239,28 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
         // events time that stage alone (same results: the order only
         // changes which link cells the dense pass skips).
         const cudaStream_t ds = serial ? st : h->side;
-        if (!serial) {
+        if (!serial && !merged) {
             FFS_CK(cudaEventRecord(h->fork, st));
             FFS_CK(cudaStreamWaitEvent(h->side, h->fork, 0));
         }
-        {
+        if (!merged) {
             StageTimer t(h, 0, ds);
             FFS_CK((launch_detect_links<DIM, T>(g, words, h->lt, sa, sc, ds)));
         }
-        if (!serial) FFS_CK(cudaEventRecord(h->join, h->side));
+        if (!serial && !merged) FFS_CK(cudaEventRecord(h->join, h->side));
     }
     {
         StageTimer t(h, 1, st);
-        if (DIM == 2) FFS_CK(launch_dense2d<T>(g, st));
+        const DetectArgs d{words, h->lt, sa, sc};
+        if constexpr (DIM == 2) FFS_CK(launch_dense2d<T>(g, st, merged ? &d : nullptr));
         else FFS_CK(launch_dense3d<T>(g, st));
     }
     if (surf) {
-        if (!serial) FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
+        if (!serial && !merged) FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
         const bool fold = (long long)sa.nv * DIM <= kFoldForcesMax;
         {
             StageTimer t(h, 2, st);
-            FFS_CK((launch_link_cells<DIM, T>(g, words, h->lt, sa, sc, st, fold)));
+            FFS_CK((launch_link_cells<DIM, T>(g, words, h->lt, sa, sc, st, fold, merged)));
         }
         if (!fold) {
             StageTimer t(h, 3, st);
@@ -788,6 +794,8 @@ template <int DIM, typename T> ffs_status noalloc_impl(ffs_lbm *h, const ffs_sur
     StepScalars sc{h->cl, h->ct, h->cf};
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);
     LinkTable lt;
+    bool merged = false; // detection in the dense pass's launch, as in step_impl
+    if constexpr (DIM == 2) merged = surf && dense2d_detects<T>(g);
     if (surf) {
         lt.cap = kNoallocSlots;
         lt.keys = reinterpret_cast<uint32_t *>(base + kNoallocKeysOff);
@@ -802,17 +810,20 @@ template <int DIM, typename T> ffs_status noalloc_impl(ffs_lbm *h, const ffs_sur
         FFS_CK(cudaMemsetAsync(lt.acc, 0, sizeof(long long) * (size_t)s->num_vertices * DIM, st));
         // detection on the grid's side stream, beside the dense pass, as in
         // step_impl (the streams and events exist since the grid was created)
-        FFS_CK(cudaEventRecord(h->fork, st));
-        FFS_CK(cudaStreamWaitEvent(h->side, h->fork, 0));
-        FFS_CK((launch_detect_links<DIM, T>(g, words, lt, sa, sc, h->side)));
-        FFS_CK(cudaEventRecord(h->join, h->side));
+        if (!merged) {
+            FFS_CK(cudaEventRecord(h->fork, st));
+            FFS_CK(cudaStreamWaitEvent(h->side, h->fork, 0));
+            FFS_CK((launch_detect_links<DIM, T>(g, words, lt, sa, sc, h->side)));
+            FFS_CK(cudaEventRecord(h->join, h->side));
+        }
     }
-    if (DIM == 2) FFS_CK(launch_dense2d<T>(g, st));
+    const DetectArgs d{words, lt, sa, sc};
+    if constexpr (DIM == 2) FFS_CK(launch_dense2d<T>(g, st, merged ? &d : nullptr));
     else FFS_CK(launch_dense3d<T>(g, st));
     if (surf) {
-        FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
+        if (!merged) FFS_CK(cudaStreamWaitEvent(st, h->join, 0));
         const bool fold = (long long)sa.nv * DIM <= kFoldForcesMax;
-        FFS_CK((launch_link_cells<DIM, T>(g, words, lt, sa, sc, st, fold)));
+        FFS_CK((launch_link_cells<DIM, T>(g, words, lt, sa, sc, st, fold, merged)));
         if (!fold) FFS_CK(launch_finalize_forces<DIM>(lt, sa, h->cf, st));
     }
     h->cur ^= 1;

@@ -434,6 +434,33 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // waits until at most N of this thread's committed groups are still in flight
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// Programmatic dependent launch: the kernel is scheduled while its predecessor
+// in the stream still runs (once every block of that one has started), and
+// waits in after_predecessor() for it to finish and its writes to be visible;
+// this hides the launch and ramp-up between two short kernels.  A kernel
+// launched this way calls after_predecessor() before it touches memory, and
+// lets its own successor in at once (a successor that was launched in the
+// plain way is not affected).
+__device__ __forceinline__ void after_predecessor()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), int grid, int block, cudaStream_t st, Args &&...args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.stream = st;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, Params(args)...);
+}
+
 template <typename T> struct GridArgs {
     int nx, ny, nz;
     uint32_t ncell;

@@ -170,6 +170,4 @@ __device__ __forceinline__ void dense2d_tile(const GridArgs<T> &g, int x0, int y
     dense2d_tile_loaded<T, HALF, TX, TY>(g, x0, y0, sp, raw, [] {});
 }
 
-template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStream_t s);
-
 } // namespace fflbm

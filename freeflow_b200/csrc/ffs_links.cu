@@ -15,7 +15,7 @@
 //               cell gets a LINK bit in its flag byte, so the dense kernels
 //               skip it.  Nothing proportional to the grid is touched.
 //   link cells  one warp per D3Q27 link-owning cell, lane i = direction i (half a
-//               warp per D2Q9 cell): wall
+//               warp per D2Q9 cell, or four lanes in the serving pool): wall
 //               bounce-back, moving-wall reconstruction with the momentum
 //               exchange force, or the ordinary pull (reconstructing the
 //               neighbour's population from its moments).  The warp reduces
@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(256, 5) link_cells_kernel(GridArgs<T> g, uint3
     const int lane = threadIdx.x & (G - 1);
     const uint32_t group = (threadIdx.x & 31) / G;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    after_predecessor();
     const LinkItems items(lt);
     const uint32_t n = items.n;
     // consecutive cells go to different CTAs: a few cells spread over the SMs
@@ -427,28 +428,27 @@ cudaError_t launch_detect_links(const GridArgs<T> &g, uint32_t *flag_words, cons
 }
 
 template <int DIM, typename T, bool HALF, bool FOLD>
-static void launch_link_cells_as(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
-                                 const StepScalars &sc, cudaStream_t st)
-{
-    link_cells_kernel<DIM, T, HALF, FOLD>
-        <<<resident_grid<link_cells_kernel<DIM, T, HALF, FOLD>>(256), 256, 0, st>>>(g, flag_words, lt, s, sc);
-}
-
-template <int DIM, typename T>
-cudaError_t launch_link_cells(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
-                              const StepScalars &sc, cudaStream_t st, bool fold_forces)
+static cudaError_t launch_link_cells_as(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
+                                        const StepScalars &sc, cudaStream_t st, bool chained)
 {
     // persistent warps over the device-side count, one wave: as many CTAs of
     // 8 warps as are resident together (a CTA beyond that would run its fixed
     // share of the cells after the others finish)
-    if (g.half_pops) {
-        if (fold_forces) launch_link_cells_as<DIM, T, true, true>(g, flag_words, lt, s, sc, st);
-        else launch_link_cells_as<DIM, T, true, false>(g, flag_words, lt, s, sc, st);
-    } else {
-        if (fold_forces) launch_link_cells_as<DIM, T, false, true>(g, flag_words, lt, s, sc, st);
-        else launch_link_cells_as<DIM, T, false, false>(g, flag_words, lt, s, sc, st);
-    }
+    const int grid = resident_grid<link_cells_kernel<DIM, T, HALF, FOLD>>(256);
+    if (chained) return launch_chained(link_cells_kernel<DIM, T, HALF, FOLD>, grid, 256, st, g, flag_words, lt, s, sc);
+    link_cells_kernel<DIM, T, HALF, FOLD><<<grid, 256, 0, st>>>(g, flag_words, lt, s, sc);
     return cudaGetLastError();
+}
+
+template <int DIM, typename T>
+cudaError_t launch_link_cells(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
+                              const StepScalars &sc, cudaStream_t st, bool fold_forces, bool chained)
+{
+    if (g.half_pops)
+        return fold_forces ? launch_link_cells_as<DIM, T, true, true>(g, flag_words, lt, s, sc, st, chained)
+                           : launch_link_cells_as<DIM, T, true, false>(g, flag_words, lt, s, sc, st, chained);
+    return fold_forces ? launch_link_cells_as<DIM, T, false, true>(g, flag_words, lt, s, sc, st, chained)
+                       : launch_link_cells_as<DIM, T, false, false>(g, flag_words, lt, s, sc, st, chained);
 }
 
 template <int DIM>
@@ -483,7 +483,7 @@ cudaError_t launch_reset_links(const LinkTable &lt, uint32_t *flag_words, cudaSt
     template cudaError_t launch_detect_links<DIM, T>(const GridArgs<T> &, uint32_t *, const LinkTable &,              \
                                                      const SurfaceArgs &, const StepScalars &, cudaStream_t);          \
     template cudaError_t launch_link_cells<DIM, T>(const GridArgs<T> &, uint32_t *, const LinkTable &,                \
-                                                   const SurfaceArgs &, const StepScalars &, cudaStream_t, bool);
+                                                   const SurfaceArgs &, const StepScalars &, cudaStream_t, bool, bool);
 FFS_INST_LINKS(2, float)
 FFS_INST_LINKS(2, __half)
 FFS_INST_LINKS(2, __nv_bfloat16)

@@ -65,14 +65,28 @@ struct StepScalars {
 // fixed-point scale of the per-vertex force sums
 constexpr double kForceScale = 4294967296.0; // 2^32
 
+// The D2Q9 dense pass (ffs_dense2d.cu).  With `detect`, the same launch does
+// launch_detect_links's work in blocks of its own; only grids for which
+// dense2d_detects() says so can.
+struct DetectArgs {
+    uint32_t *flag_words;
+    LinkTable lt;
+    SurfaceArgs s;
+    StepScalars sc;
+};
+template <typename T> bool dense2d_detects(const GridArgs<T> &g);
+template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStream_t s, const DetectArgs *detect = nullptr);
+
 template <int DIM, typename T>
 cudaError_t launch_detect_links(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
                                 const StepScalars &sc, cudaStream_t st);
 // With fold_forces, the last CTA also does launch_finalize_forces's work
 // (the caller launches no finalize kernel); lt.done must be allocated.
+// chained: the stream's last operation is the launch of the dense pass with
+// detection in it, which lets this kernel in early (launch_chained).
 template <int DIM, typename T>
 cudaError_t launch_link_cells(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt, const SurfaceArgs &s,
-                              const StepScalars &sc, cudaStream_t st, bool fold_forces = false);
+                              const StepScalars &sc, cudaStream_t st, bool fold_forces = false, bool chained = false);
 template <int DIM>
 cudaError_t launch_finalize_forces(const LinkTable &lt, const SurfaceArgs &s, double cf, cudaStream_t st);
 template <int DIM>

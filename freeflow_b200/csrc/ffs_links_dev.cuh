@@ -394,9 +394,16 @@ __device__ __forceinline__ void add_forces_warp(long long *acc, bool active, uin
         }
 }
 
-// Lanes per link cell: a D3Q27 cell takes a whole warp, a D2Q9 cell half of
-// one, so a warp updates two D2Q9 cells at once.
+// Lanes per link cell.  A D3Q27 cell takes a whole warp, one lane per
+// direction.  A D2Q9 cell takes 16 lanes of one direction each where a step
+// has a few hundred link cells (one grid: its time is the chain of one cell's
+// loads), and 4 lanes of up to three directions where it has tens of
+// thousands (the serving pool: its time is the instructions, 390 per lane and
+// cell, most of them the cell's own coefficients and idle lanes).  On one
+// 1200 x 400 grid 4 lanes cost 2 us a step against 16; in the pool they took
+// the link cells of 64 episodes from 25.6 to 13 us a substep.
 template <int DIM> constexpr int kLinkGroup = DIM == 2 ? 16 : 32;
+constexpr int kPoolLinkGroup = 4;
 
 // Update of one link-owning D3Q27 cell by one warp (lane i = direction i;
 // D2Q9: link_cell_update2): wall bounce-back, moving-wall

@@ -9,15 +9,16 @@
 // eviction and stepping never allocate device memory.
 //
 // Stepping: all admitted episodes advance together.  One control step is one
-// CUDA-graph launch of `substeps` x {kinematics, link detection, dense pass,
-// link cells, force reduction} plus the output kernel; every kernel covers
-// all episodes and reads their number from the device-side active table, so
-// the graph is captured once per (tile shape, starting buffer parity) and
+// CUDA-graph launch: the first substep's kinematics, then `substeps` x {dense
+// pass with link detection, link cells, force reduction with the next
+// substep's kinematics}, then the output kernel; every kernel covers all
+// episodes and reads their number from the device-side active table, so
+// the graph is captured once per (rows per unit, starting buffer parity) and
 // reused for every mix.  The active table is re-uploaded only after the mix
 // changed; the per-step parameters (actions, wave phases) are one upload.
 //
-// Work unit of the dense pass: ffs_pool_tune times the candidate units
-// (tiles and row-marching strips, kPoolShapes) on the current mix (CUDA
+// Work unit of the dense pass: ffs_pool_tune times the candidate units (march
+// units of 64 columns and kPoolRows rows) on the current mix (CUDA
 // events, a warm launch then five timed ones each) and keeps the fastest.
 // Every unit gives the same bits, so the choice changes only the speed.  It
 // runs by itself on the first advance and again when the number of cells has
@@ -44,6 +45,7 @@
 #include "ffs_pool.h"
 #include "ffs_common.cuh"
 #include "ffs_links.cuh"
+#include "ffs_march2d.cuh"
 #include "ffs_pool.cuh"
 
 using namespace fflbm;
@@ -190,6 +192,7 @@ struct ffs_pool {
     PoolOutput *d_out = nullptr, *h_out[2] = {};
     LinkTable lt;
     uint32_t *owner = nullptr;
+    uint32_t *unit_next = nullptr; // next march unit of the dense pass, behind the link counts; zeroed by kinematics
     int shape = 1;
     bool act_dirty = true;
     int64_t tuned_cells = 0; // cells of the mix at the last tuning (0: never)
@@ -205,10 +208,10 @@ struct ffs_pool {
     int last = 0;             // buffer of the latest control step
     int64_t advances = 0, graph_builds = 0;
     int sms = 0;              // SMs of the device, queried at creation
-    int grid_dense[kPoolNumShapes] = {};
-    int grid_link = 0;        // resident CTAs of the link-cell kernel (one wave)
+    int grid_dense = 0;       // resident CTAs of the dense kernel
     float *stage = nullptr;   // ffs_pool_get_moments' AoS copy of one episode, kept (at most the largest episode's size)
     size_t stage_bytes = 0;
+    int grid_link = 0;        // resident CTAs of the link-cell kernel (one wave)
 };
 
 namespace {
@@ -226,12 +229,12 @@ int64_t mix_cells(const ffs_pool *p)
 void build_active(ffs_pool *p)
 {
     PoolActive &A = *p->h_act;
-    const PoolTileShape sh = kPoolShapes[p->shape];
+    const int rows = kPoolRows[p->shape];
     A.n = (uint32_t)p->order.size();
     A.tile_prefix[0] = A.elem_prefix[0] = A.vert_prefix[0] = 0;
     for (size_t a = 0; a < p->order.size(); ++a) {
         const Slot &s = p->slots[p->order[a]];
-        const uint32_t tx = (uint32_t)((s.nx + sh.tx - 1) / sh.tx), ty = (uint32_t)((s.ny + sh.ty - 1) / sh.ty);
+        const uint32_t tx = (uint32_t)march2::windows(s.nx), ty = (uint32_t)march2::chunks(s.ny, rows);
         A.slot[a] = (uint32_t)p->order[a];
         A.tiles_x[a] = tx;
         A.tile_prefix[a + 1] = A.tile_prefix[a] + tx * ty;
@@ -276,18 +279,20 @@ ffs_status wait_idle(ffs_pool *p)
 template <typename T> ffs_status capture(ffs_pool *p, int shape, int parity, cudaGraphExec_t *out)
 {
     const int S = p->d.substeps;
-    const int g_kin = p->sms * 4, g_det = p->sms * 4, g_link = p->grid_link, g_fin = p->sms * 2;
+    const int g_kin = p->sms * 4, g_link = p->grid_link, g_fin = p->sms * 2;
     cudaGraph_t graph = nullptr;
     POOL_CK(cudaStreamBeginCapture(p->st, cudaStreamCaptureModeThreadLocal));
     cudaError_t err = cudaSuccess;
     int par = parity;
+    err = launch_pool_kinematics(p->d_eps, p->d_prm, p->d_act, p->unit_next, g_kin, p->st);
     for (int j = 0; j < S && err == cudaSuccess; ++j) {
-        if ((err = launch_pool_kinematics(p->d_eps, p->d_prm, p->d_act, j, g_kin, p->st)) != cudaSuccess) break;
-        if ((err = launch_pool_detect<T>(p->d_eps, p->d_act, p->lt, p->owner, par, g_det, p->st)) != cudaSuccess) break;
-        if ((err = launch_pool_dense<T>(p->d_eps, p->d_act, par, shape, p->grid_dense[shape], p->st)) != cudaSuccess)
+        if ((err = launch_pool_dense<T>(p->d_eps, p->d_act, p->lt, p->owner, p->unit_next, true, par, shape, p->grid_dense,
+                                        p->st)) != cudaSuccess)
             break;
         if ((err = launch_pool_link_cells<T>(p->d_eps, p->lt, p->owner, par, g_link, p->st)) != cudaSuccess) break;
-        if ((err = launch_pool_finalize(p->d_eps, p->d_act, p->lt, g_fin, p->st)) != cudaSuccess) break;
+        if ((err = launch_pool_finalize(p->d_eps, p->d_prm, p->d_act, p->lt, p->unit_next, j + 1 < S ? j + 1 : 0, g_fin,
+                                        p->st)) != cudaSuccess)
+            break;
         par ^= 1;
     }
     if (err == cudaSuccess) err = launch_pool_outputs(p->d_eps, p->d_act, p->d_out, S, p->st);
@@ -300,7 +305,7 @@ template <typename T> ffs_status capture(ffs_pool *p, int shape, int parity, cud
     return FFS_OK;
 }
 
-// FFS_POOL_SHAPE pins the dense work unit (an index into kPoolShapes) for
+// FFS_POOL_SHAPE pins the dense work unit (an index into kPoolRows) for
 // tests that check every unit; -1 when unset or out of range.
 static int pinned_shape()
 {
@@ -322,10 +327,12 @@ template <typename T> ffs_status tune_impl(ffs_pool *p)
         if (r != FFS_OK) return r;
         // the dense pass reads the current buffer and writes the other one,
         // which the next real step overwrites: repeating it changes no state
-        POOL_CK((launch_pool_dense<T>(p->d_eps, p->d_act, p->parity, sh, p->grid_dense[sh], p->st)));
-        POOL_CK(cudaEventRecord(p->ev0, p->st));
-        for (int r2 = 0; r2 < 5; ++r2)
-            POOL_CK((launch_pool_dense<T>(p->d_eps, p->d_act, p->parity, sh, p->grid_dense[sh], p->st)));
+        for (int r2 = -1; r2 < 5; ++r2) {
+            if (r2 == 0) POOL_CK(cudaEventRecord(p->ev0, p->st));
+            POOL_CK(cudaMemsetAsync(p->unit_next, 0, sizeof(uint32_t), p->st));
+            POOL_CK((launch_pool_dense<T>(p->d_eps, p->d_act, p->lt, p->owner, p->unit_next, false, p->parity, sh,
+                                          p->grid_dense, p->st)));
+        }
         POOL_CK(cudaEventRecord(p->ev1, p->st));
         POOL_CK(cudaEventSynchronize(p->ev1));
         float ms = 0.0f;
@@ -457,21 +464,18 @@ ffs_status ffs_pool_create(const ffs_pool_desc *desc, ffs_pool **out)
     if ((e = cudaMalloc(&p->lt.keys, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link keys");
     if ((e = cudaMalloc(&p->lt.links, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "links");
     if ((e = cudaMalloc(&p->lt.list, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link list");
-    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t) * kCountWords)) != cudaSuccess) return bail(e, "link count");
+    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t) * (kCountWords + 1))) != cudaSuccess) return bail(e, "link count");
     if ((e = cudaMalloc(&p->owner, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link owner");
     if ((e = cudaMemset(p->lt.keys, 0, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemset(p->lt.links, 0xFF, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "memset");
-    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t) * kCountWords)) != cudaSuccess) return bail(e, "memset");
+    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t) * (kCountWords + 1))) != cudaSuccess) return bail(e, "memset");
+    p->unit_next = p->lt.count + kCountWords;
     p->lt.acc = nullptr; // per-episode accumulators live in the arena
     p->lt.acc_cap = 0;
-    for (int sh = 0; sh < kPoolNumShapes; ++sh) {
-        int b = 1;
-        switch (d.storage) {
-        case FFS_STORAGE_F32: b = pool_dense_blocks_per_sm<float>(sh); break;
-        case FFS_STORAGE_F16: b = pool_dense_blocks_per_sm<__half>(sh); break;
-        default: b = pool_dense_blocks_per_sm<__nv_bfloat16>(sh); break;
-        }
-        p->grid_dense[sh] = p->sms * b;
+    switch (d.storage) {
+    case FFS_STORAGE_F32: p->grid_dense = p->sms * pool_dense_blocks_per_sm<float>(); break;
+    case FFS_STORAGE_F16: p->grid_dense = p->sms * pool_dense_blocks_per_sm<__half>(); break;
+    default: p->grid_dense = p->sms * pool_dense_blocks_per_sm<__nv_bfloat16>(); break;
     }
     switch (d.storage) {
     case FFS_STORAGE_F32: p->grid_link = p->sms * pool_link_cells_blocks_per_sm<float>(); break;
@@ -812,16 +816,16 @@ ffs_status ffs_pool_get_info(const ffs_pool *p, ffs_pool_info *info)
     info->free_bytes = (int64_t)p->arena.free_bytes();
     info->largest_free_bytes = (int64_t)p->arena.largest();
     info->active_episodes = (int)p->order.size();
-    const PoolTileShape sh = kPoolShapes[p->shape];
+    const int rows = kPoolRows[p->shape];
     int64_t tiles = 0;
     for (int si : p->order) {
         const Slot &s = p->slots[si];
-        tiles += (int64_t)((s.nx + sh.tx - 1) / sh.tx) * ((s.ny + sh.ty - 1) / sh.ty);
+        tiles += (int64_t)march2::windows(s.nx) * march2::chunks(s.ny, rows);
     }
     info->tiles = (int)tiles;
-    info->tile_x = sh.tx;
-    info->tile_y = sh.ty;
-    info->strip = sh.strip ? 1 : 0;
+    info->tile_x = march2::kWindow;
+    info->tile_y = rows;
+    info->strip = 1;
     info->advances = p->advances;
     info->graph_builds = p->graph_builds;
     info->cells = mix_cells(p);

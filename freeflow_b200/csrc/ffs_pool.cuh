@@ -97,35 +97,81 @@ __host__ __device__ inline void swimmer_vertex(float rx, float ry, float amp, fl
 #undef FFS_ADD
 #undef FFS_SUB
 
-// Work units of the batched dense pass (the autotuner's candidates): tiles
-// of tx x ty cells, one thread per cell (pool_dense_kernel), or strips of tx
-// columns and ty rows walked row by row by tx + 2 threads (pool_strip_kernel).
-struct PoolTileShape {
-    int tx, ty;
-    bool strip;
-};
+// Work units of the batched dense pass (the autotuner's candidates): march
+// units (ffs_march2d.cuh) of 64 columns and so many rows.
 constexpr int kPoolNumShapes = 8;
-constexpr PoolTileShape kPoolShapes[kPoolNumShapes] = {{32, 4, false},  {32, 8, false},  {64, 4, false},
-                                                       {32, 16, false}, {64, 8, false},  {62, 32, true},
-                                                       {126, 32, true}, {126, 64, true}};
+constexpr int kPoolRows[kPoolNumShapes] = {1, 2, 3, 4, 6, 8, 11, 14};
 
-cudaError_t launch_pool_kinematics(const PoolEpisode *eps, const PoolParams *prm, const PoolActive *act, int substep,
-                                   int grid, cudaStream_t st);
+// Index of the active entry whose range [prefix[i], prefix[i+1]) holds t.
+__device__ __forceinline__ int owner_of(const uint32_t *prefix, int n, uint32_t t)
+{
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (prefix[mid] <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// What the step's kernels take of an episode, its buffers in the order that
+// this substep reads and writes them.
+template <typename T> __device__ __forceinline__ GridArgs<T> episode_args(const PoolEpisode &e, int parity)
+{
+    GridArgs<T> g;
+
+    g.nx = e.nx;
+    g.ny = e.ny;
+    g.nz = 1;
+    g.ncell = e.ncell;
+    g.periodic = 0;
+    g.half_pops = 0;
+    g.wall_stream = 0;
+    g.omega = e.omega;
+    g.codec = e.codec;
+    g.src = static_cast<const T *>(e.mom[parity]);
+    g.dst = static_cast<T *>(e.mom[parity ^ 1]);
+    g.flags = e.flags;
+    g.wallmask = e.wallmask;
+    g.status = e.status;
+    // the arena is device memory: plain global accesses
+    __builtin_assume(__isGlobal(g.src));
+    __builtin_assume(__isGlobal(g.dst));
+    __builtin_assume(__isGlobal(g.flags));
+    __builtin_assume(__isGlobal(g.wallmask));
+    return g;
+}
+
+__device__ __forceinline__ SurfaceArgs episode_surface(const PoolEpisode &e)
+{
+    SurfaceArgs s{};
+    s.V = e.V;
+    s.U = e.U;
+    s.E = e.elements;
+    s.nv = e.nv;
+    s.ne = e.ne;
+    s.forces = nullptr;
+    s.forces64 = nullptr;
+    return s;
+}
+
+// A control step is kinematics, then per substep the dense pass with link
+// detection in it, the link cells and the force reduction, which also moves
+// the surfaces to the next substep (`next`, 0 on the last), then the outputs.
+cudaError_t launch_pool_kinematics(const PoolEpisode *eps, const PoolParams *prm, const PoolActive *act,
+                                   uint32_t *unit_next, int grid, cudaStream_t st);
 template <typename T>
-cudaError_t launch_pool_detect(const PoolEpisode *eps, const PoolActive *act, const LinkTable &lt, uint32_t *owner,
-                               int parity, int grid, cudaStream_t st);
+cudaError_t launch_pool_dense(const PoolEpisode *eps, const PoolActive *act, const LinkTable &lt, uint32_t *owner,
+                              uint32_t *unit_next, bool detect, int parity, int shape, int grid, cudaStream_t st);
 template <typename T>
-cudaError_t launch_pool_dense(const PoolEpisode *eps, const PoolActive *act, int parity, int shape, int grid,
-                              cudaStream_t st);
-template <typename T>
-int pool_dense_blocks_per_sm(int shape);
+int pool_dense_blocks_per_sm();
 template <typename T>
 int pool_link_cells_blocks_per_sm();
 template <typename T>
 cudaError_t launch_pool_link_cells(const PoolEpisode *eps, const LinkTable &lt, const uint32_t *owner, int parity,
                                    int grid, cudaStream_t st);
-cudaError_t launch_pool_finalize(const PoolEpisode *eps, const PoolActive *act, const LinkTable &lt, int grid,
-                                 cudaStream_t st);
+cudaError_t launch_pool_finalize(const PoolEpisode *eps, const PoolParams *prm, const PoolActive *act,
+                                 const LinkTable &lt, uint32_t *unit_next, int next, int grid, cudaStream_t st);
 cudaError_t launch_pool_outputs(const PoolEpisode *eps, const PoolActive *act, PoolOutput *out, int substeps,
                                 cudaStream_t st);
 
