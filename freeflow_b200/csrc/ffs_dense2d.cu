@@ -35,23 +35,23 @@ __global__ void __launch_bounds__(D2::kThreads) dense2d_kernel(GridArgs<T> g)
     dense2d_tile<T, HALF>(g, blockIdx.x * D2::kTX, blockIdx.y * D2::kTY, sp);
 }
 
-// The first `ndetect` CTAs detect the surface's links (four elements a warp at
-// a time), the others march.  A launch of its own for detection, on a second
+// The first `ndetect` CTAs detect the surface's links (`lanes` lanes an
+// element), the others march.  A launch of its own for detection, on a second
 // stream with events around it, cost more than detection itself on grids of
 // this size; which link cells the march skips (it reads their LINK bit while
 // detection sets it) does not matter, because the link-cell kernel rewrites
 // every link cell afterwards.
 template <typename T, bool VEC>
-__global__ void __launch_bounds__(32, kMarchWarps) march2d_kernel(GridArgs<T> g, int rows, int ndetect, DetectArgs d)
+__global__ void __launch_bounds__(32, kMarchWarps) march2d_kernel(GridArgs<T> g, int rows, int ndetect, int lanes, DetectArgs d)
 {
     __shared__ march2::Ends ends;
     after_predecessor();
     if ((int)blockIdx.x < ndetect) {
         uint32_t *queue = reinterpret_cast<uint32_t *>(&ends);
         static_assert(sizeof(ends) >= 64 * sizeof(uint32_t), "the exact test's queue fits");
-        const int group = threadIdx.x >> 3;
-        for (long long e = (long long)blockIdx.x * 4; e < d.s.ne; e += (long long)ndetect * 4)
-            detect_elements2_warp<T>(g, d.flag_words, d.lt, d.s, d.sc, e + group, e + group < d.s.ne, queue);
+        const int per = 32 / lanes, group = (int)threadIdx.x / lanes;
+        for (long long e = (long long)blockIdx.x * per; e < d.s.ne; e += (long long)ndetect * per)
+            detect_elements2_warp<T>(g, d.flag_words, d.lt, d.s, d.sc, e + group, e + group < d.s.ne, lanes, queue);
         return;
     }
     const int W = march2::windows(g.nx), u = (int)blockIdx.x - ndetect;
@@ -99,10 +99,11 @@ template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStrea
     }
     const int rows = march_rows(g.nx, g.ny);
     const int units = march2::windows(g.nx) * march2::chunks(g.ny, rows);
-    const int nd = detect ? (int)std::min<long long>(((long long)detect->s.ne + 3) / 4, (long long)device_sms() * 32) : 0;
+    const int lanes = detect ? detect_lanes2(detect->s.ne, device_sms()) : 32, per = 32 / lanes;
+    const int nd = detect ? (int)std::min<long long>(((long long)detect->s.ne + per - 1) / per, (long long)device_sms() * 32) : 0;
     const DetectArgs d = detect ? *detect : DetectArgs{};
-    if (g.nx % 2 == 0) march2d_kernel<T, true><<<units + nd, 32, 0, s>>>(g, rows, nd, d);
-    else march2d_kernel<T, false><<<units + nd, 32, 0, s>>>(g, rows, nd, d);
+    if (g.nx % 2 == 0) march2d_kernel<T, true><<<units + nd, 32, 0, s>>>(g, rows, nd, lanes, d);
+    else march2d_kernel<T, false><<<units + nd, 32, 0, s>>>(g, rows, nd, lanes, d);
     return cudaGetLastError();
 }
 
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(32, kMarchWarps)
             const PoolEpisode &e = eps[s];
             detect_elements2_warp<T>(episode_args<T>(e, parity), reinterpret_cast<uint32_t *>(e.flags), lt,
                                      episode_surface(e), StepScalars{e.cl, e.ct, e.cf},
-                                     (long long)(ge - act->elem_prefix[a]), mine < elements,
+                                     (long long)(ge - act->elem_prefix[a]), mine < elements, 8,
                                      reinterpret_cast<uint32_t *>(&ends), e.cell_base, owner, s);
         } else {
             const int a = owner_of(act->tile_prefix, n, t - first);

@@ -75,7 +75,9 @@ __device__ __forceinline__ void clear_counts(const LinkTable &lt)
 // Finds or claims the cell's slot and keeps the smallest key of direction l.
 // The table key is key_base + cell + 1: one table can serve many grids whose
 // cells are numbered from distinct bases; the claiming thread tags the slot
-// with owner_id in `owner` when that array is given.
+// with owner_id in `owner` when that array is given.  A lane waits for one or
+// two round trips to L2 here (the compare-and-swap, and the list position of a
+// new slot), which is most of a small surface's detection time.
 template <int Q>
 __device__ __forceinline__ void insert_link(const LinkTable &lt, uint32_t *flag_words, uint32_t cell, int l,
                                             unsigned long long key, uint32_t *status, uint32_t key_base = 0,
@@ -84,22 +86,16 @@ __device__ __forceinline__ void insert_link(const LinkTable &lt, uint32_t *flag_
     const uint32_t tkey = key_base + cell + 1;
     uint32_t slot = hash_cell(tkey - 1) & (lt.cap - 1);
     for (uint32_t probe = 0; probe < lt.cap; ++probe) {
-        uint32_t cur = lt.keys[slot];
-        if (cur == 0) {
-            uint32_t old = atomicCAS(lt.keys + slot, 0u, tkey);
-            if (old == 0) {
+        const uint32_t old = atomicCAS(lt.keys + slot, 0u, tkey);
+        if (old == 0u || old == tkey) {
+            atomicMin(lt.links + (size_t)slot * Q + l, key);
+            if (old == 0u) {
                 const uint32_t seg = slot >> lt.seg_shift;
                 const uint32_t pos = atomicAdd(lt.count + seg * kCountStride, 1u);
-                lt.list[(seg << lt.seg_shift) + pos] = slot;
                 if (owner) owner[slot] = owner_id;
                 set_link_bit(flag_words, cell, true);
-                cur = tkey;
-            } else {
-                cur = old;
+                lt.list[(seg << lt.seg_shift) + pos] = slot;
             }
-        }
-        if (cur == tkey) {
-            atomicMin(lt.links + (size_t)slot * Q + l, key);
             return;
         }
         slot = (slot + 1) & (lt.cap - 1);
@@ -226,9 +222,10 @@ __device__ __forceinline__ void detect_element2_warp(const GridArgs<T> &g, uint3
     __syncwarp();
 }
 
-// D2Q9 link detection of four segments by one warp, eight lanes (the eight
-// directions) each: the lane group's element e (when `valid`), of a surface
-// and a grid that may differ from group to group.
+// D2Q9 link detection of one or four segments by one warp, `lanes` = 32 or 8
+// lanes each (the eight directions, and the lines of one direction dealt out
+// to the lanes that share it): the lane group's element e (when `valid`), of a
+// surface and a grid that may differ from group to group.
 //
 // A link segment x -> x - c lies on one of the lattice lines parallel to c,
 // and such a line meets the element's line in one point, so a lane looks only
@@ -251,18 +248,18 @@ __device__ __forceinline__ void detect_element2_warp(const GridArgs<T> &g, uint3
 template <typename T>
 __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint32_t *flag_words, const LinkTable &lt,
                                                       const SurfaceArgs &s, const StepScalars &sc, long long e, bool valid,
-                                                      uint32_t *wq, uint32_t key_base = 0, uint32_t *owner = nullptr,
-                                                      uint32_t owner_id = 0)
+                                                      int lanes, uint32_t *wq, uint32_t key_base = 0,
+                                                      uint32_t *owner = nullptr, uint32_t owner_id = 0)
 {
     constexpr int Q = 9;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, first = lane & ~(lanes - 1);
     const unsigned full = 0xffffffffu;
     uint32_t va = 0, vb = 0;
     if (valid) {
         va = s.E[2 * e];
         vb = s.E[2 * e + 1];
         if (va >= (uint32_t)s.nv || vb >= (uint32_t)s.nv) {
-            if ((lane & 7) == 0) atomicOr(g.status, kStatusBadElement);
+            if (lane == first) atomicOr(g.status, kStatusBadElement);
             valid = false;
         }
     }
@@ -313,7 +310,7 @@ __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint
             const float slack = reach ? 1.2f * margin * fabsf(inv) * inv_cl + 2e-3f : 1e9f;
             const float from = (ck > 0 ? 0.0f : -1.0f) - slack, to = (ck > 0 ? 1.0f : 0.0f) + slack;
             const float klo = (float)lk, khi = (float)hk;
-            for (; q <= qend; ++q) {
+            for (q += (lane - first) >> 3; q <= qend; q += lanes >> 3) {
                 const float sk = k4 - gq * ((float)q - q4);
                 int k = (int)ceilf(fmaxf(sk + from, klo));
                 const int kend = (int)floorf(fminf(sk + to, khi));
@@ -336,7 +333,7 @@ __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint
         }
     }
     // nearly vertical elements: the whole warp takes them one by one
-    for (unsigned left = __ballot_sync(full, plain && (lane & 7) == 0); left; left &= left - 1) {
+    for (unsigned left = __ballot_sync(full, plain && lane == first); left; left &= left - 1) {
         const int from = __ffs(left) - 1;
         auto of = [&](auto v) {
             decltype(v) r;
