@@ -38,7 +38,7 @@ __global__ void pool_kinematics_kernel(const PoolEpisode *eps, const PoolParams 
                                        uint32_t *unit_next)
 {
     after_predecessor();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *unit_next = 0; // the next dense pass counts from it
+    if (blockIdx.x == 0 && threadIdx.x < 2) unit_next[threadIdx.x] = 0; // the next dense pass counts from them
     const int n = (int)act->n;
     if (n == 0) return;
     const uint32_t total = act->vert_prefix[n];
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(256) pool_finalize_kernel(const PoolEpisode *e
 {
     __shared__ double red[4][8];
     after_predecessor();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *unit_next = 0; // the next dense pass counts from it
+    if (blockIdx.x == 0 && threadIdx.x < 2) unit_next[threadIdx.x] = 0; // the next dense pass counts from them
     const int n = (int)act->n;
     if (blockIdx.x == 0) clear_counts(lt);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

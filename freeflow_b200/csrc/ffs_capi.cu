@@ -43,6 +43,7 @@ struct ffs_lbm {
     Codec codec{};
     LinkTable lt;
     float *staging = nullptr; // ncell * NM floats, allocated on first host transfer
+    uint32_t *feeders = nullptr;   // [1 + feeders_cap] cells that feed outlets (GridArgs::feeders)
     uint32_t *fill_bits = nullptr; // D3Q27 solid fill: one parity bit per cell, zero between calls
     // link detection runs on `side` while the dense pass runs on the caller's
     // stream; fork/join order them
@@ -91,6 +92,15 @@ uint32_t next_pow2(uint64_t v)
     return (uint32_t)std::min<uint64_t>(p, 1ull << 31);
 }
 
+// Feeders of outlets a grid's list holds: as many as outlets on all its faces
+// have.  (With more, from outlet nodes inside the grid, the step looks for them
+// in the flag bytes.)
+uint32_t feeders_cap(int dim, int nx, int ny, int nz)
+{
+    const int64_t x = nx, y = ny, z = nz;
+    return (uint32_t)std::min<int64_t>(dim == 2 ? 2 * (x + y) : 2 * (x * y + y * z + x * z), x * y * (dim == 2 ? 1 : z));
+}
+
 template <typename T> GridArgs<T> args(ffs_lbm *h)
 {
     GridArgs<T> g;
@@ -101,6 +111,9 @@ template <typename T> GridArgs<T> args(ffs_lbm *h)
     g.periodic = h->d.periodic_mask;
     g.half_pops = h->dim == 2 ? h->d.ref_half_populations : 0;
     g.wall_stream = h->dim == 2 ? h->d.ref_2d_wall_stream : 0;
+    g.feed = kBitOutletSrc;
+    g.feeders = h->feeders;
+    g.feeders_cap = feeders_cap(h->dim, h->d.nx, h->d.ny, h->d.nz);
     g.omega = h->omega;
     g.codec = h->codec;
     g.src = static_cast<const T *>(h->mom[h->cur]);
@@ -219,6 +232,7 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
 {
     GridArgs<T> g = args<T>(h);
     const bool surf = sa.ne > 0;
+    if (surf) g.feed = 0;
     StepScalars sc{h->cl, h->ct, h->cf};
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);
     const bool serial = h->profiling == 2;
@@ -234,10 +248,11 @@ template <int DIM, typename T> ffs_status step_impl(ffs_lbm *h, const SurfaceArg
         }
         // Link detection and the dense pass overlap: the dense pass skips
         // cells whose LINK bit it sees, but any link cell it does update is
-        // rewritten by link_cells, which runs after both.  Serial profiling
-        // runs detection on the caller's stream first, so that each stage's
-        // events time that stage alone (same results: the order only
-        // changes which link cells the dense pass skips).
+        // rewritten by link_cells, which runs after both and feeds every
+        // outlet.  Serial profiling runs detection on the caller's stream
+        // first, so that each stage's events time that stage alone (same
+        // moments and forces: the order only changes which link cells the
+        // dense pass skips).
         const cudaStream_t ds = serial ? st : h->side;
         if (!serial && !merged) {
             FFS_CK(cudaEventRecord(h->fork, st));
@@ -341,8 +356,10 @@ int which_index(const ffs_lbm *h, int which)
 
 ffs_status prepare_flags(ffs_lbm *h, cudaStream_t st)
 {
-    if (h->dim == 2) FFS_CK(launch_prepare_flags<2>(h->flags, h->wallmask, h->d.nx, h->d.ny, 1, st));
-    else FFS_CK(launch_prepare_flags<3>(h->flags, h->wallmask, h->d.nx, h->d.ny, h->d.nz, st));
+    const uint32_t cap = feeders_cap(h->dim, h->d.nx, h->d.ny, h->d.nz);
+    FFS_CK(cudaMemsetAsync(h->feeders, 0, sizeof(uint32_t), st));
+    if (h->dim == 2) FFS_CK(launch_prepare_flags<2>(h->flags, h->wallmask, h->feeders, cap, h->d.nx, h->d.ny, 1, st));
+    else FFS_CK(launch_prepare_flags<3>(h->flags, h->wallmask, h->feeders, cap, h->d.nx, h->d.ny, h->d.nz, st));
     return FFS_OK;
 }
 
@@ -423,6 +440,8 @@ ffs_status ffs_lbm_create(const ffs_lbm_desc *desc, ffs_lbm **out)
     const size_t fbytes = ((size_t)ncell + 3) & ~(size_t)3;
     if ((e = cudaMalloc(&h->flags, fbytes)) != cudaSuccess) return bail(e, "flags");
     if ((e = cudaMalloc(&h->wallmask, sizeof(uint32_t) * (size_t)ncell)) != cudaSuccess) return bail(e, "wallmask");
+    if ((e = cudaMalloc(&h->feeders, sizeof(uint32_t) * (1 + (size_t)feeders_cap(d.dim, d.nx, d.ny, nz)))) != cudaSuccess)
+        return bail(e, "feeders");
     if ((e = cudaMalloc(&h->status, sizeof(uint32_t))) != cudaSuccess) return bail(e, "status");
     if ((e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
     if ((e = cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming)) != cudaSuccess) return bail(e, "event");
@@ -453,6 +472,7 @@ ffs_status ffs_lbm_destroy(ffs_lbm *h)
     if (h->side) cudaStreamDestroy(h->side);
     cudaFree(h->mom[0]); cudaFree(h->mom[1]); cudaFree(h->flags); cudaFree(h->wallmask); cudaFree(h->status);
     cudaFree(h->staging);
+    cudaFree(h->feeders);
     cudaFree(h->fill_bits);
     free_links(h->lt);
     delete h;
@@ -790,6 +810,7 @@ template <int DIM, typename T> ffs_status noalloc_impl(ffs_lbm *h, const ffs_sur
     constexpr int Q = Lattice<DIM>::Q;
     GridArgs<T> g = args<T>(h);
     const bool surf = s && s->num_elements > 0;
+    if (surf) g.feed = 0;
     SurfaceArgs sa = surface_args(s);
     StepScalars sc{h->cl, h->ct, h->cf};
     uint32_t *words = reinterpret_cast<uint32_t *>(h->flags);

@@ -128,7 +128,8 @@ enum Flag : uint8_t {
 // The device flag byte keeps the node type in its low 5 bits and three
 // derived bits the kernels use to stay on the fast path:
 constexpr uint8_t kTypeMask = 0x1F;
-constexpr uint8_t kBitOutletSrc = 0x20; // fluid cell that feeds a neighbouring outlet node
+constexpr uint8_t kBitOutletSrc = 0x20; // fluid cell that feeds a neighbouring outlet node; on an outlet node:
+                                        // its feeder has links this step (mark_outlets)
 constexpr uint8_t kBitNearWall = 0x40;  // some neighbour x - c_i is a bounce-back node
 constexpr uint8_t kBitLink = 0x80;      // cell has moving-boundary links this step
 
@@ -148,7 +149,7 @@ enum StatusBits : uint32_t {
     kStatusLinkOverflow = 1u << 1,  // link hash table full; some links were dropped
     kStatusForceRange = 1u << 2,    // a force contribution exceeded the fixed-point range
     kStatusBadElement = 1u << 3,    // element index out of range in the surface
-    kStatusStageTimeout = 1u << 4,  // a staged plane of moments did not arrive within the wait limit
+    kStatusWaitTimeout = 1u << 4,   // a wait inside a kernel ran out (march2::Gate)
 };
 
 // A post-collision state the step cannot continue from: density not
@@ -468,12 +469,15 @@ template <typename T> struct GridArgs {
     int half_pops;           // D2Q9: round reconstructed populations to binary16 (reference tile)
     int wall_stream;         // D2Q9: walls stream their stored moments instead of bouncing back
                              // (the reference's 2D kernel, ffs_lbm_desc::ref_2d_wall_stream)
+    uint32_t feed;           // kBitOutletSrc: the dense pass feeds outlets; 0: the link-cell kernel does (ffs_outlet.cuh)
     float omega;
     Codec codec;
     const T *src;            // SoA: moment k of cell c at src[k * ncell + c]
     T *dst;
     const uint8_t *flags;
     const uint32_t *wallmask; // per-cell bounce-back direction mask (read only for near-wall cells)
+    const uint32_t *feeders; // the number of cells that feed outlets, then up to feeders_cap of them (single grids)
+    uint32_t feeders_cap;
     uint32_t *status;
 };
 

@@ -38,9 +38,9 @@ __global__ void __launch_bounds__(D2::kThreads) dense2d_kernel(GridArgs<T> g)
 // The first `ndetect` CTAs detect the surface's links (`lanes` lanes an
 // element), the others march.  A launch of its own for detection, on a second
 // stream with events around it, cost more than detection itself on grids of
-// this size; which link cells the march skips (it reads their LINK bit while
-// detection sets it) does not matter, because the link-cell kernel rewrites
-// every link cell afterwards.
+// this size.  Which link cells the march skips (it reads their LINK bit while
+// detection sets it) does not matter: the link-cell kernel rewrites every link
+// cell afterwards and feeds the outlets (ffs_outlet.cuh).
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(32, kMarchWarps) march2d_kernel(GridArgs<T> g, int rows, int ndetect, int lanes, DetectArgs d)
 {
@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(32, kMarchWarps) march2d_kernel(GridArgs<T> g,
     // the top rows start right after the bottom ones: both may feed outlets,
     // which takes a unit longer (0.5 us of a 22 us step on 1200 x 400)
     const int c = c0 == 1 ? C - 1 : c0 > 1 ? c0 - 1 : 0;
-    march2::run<T, VEC>(g, w, c * rows, min((c + 1) * rows, g.ny), ends);
+    march2::Gate gate{nullptr, 0u, false};
+    march2::run<T, VEC>(g, w, c * rows, min((c + 1) * rows, g.ny), ends, gate);
 }
 
 // Rows per unit: a unit reconstructs rows + 2 rows, a row of one warp alone
@@ -114,8 +115,14 @@ template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStrea
 // walls takes fewer (with fixed shares the slowest SM ran 35 % longer than the
 // fastest), and detection, a chain of dependent atomics that left the chip
 // idle in a launch of its own, runs beside the march.  The next unit is
-// fetched while the current one runs.  Episodes hold fewer than 2^22 cells, so
-// every moment index fits in 32 bits.
+// fetched while the current one runs.  Every unit, a CTA's first too, comes
+// from the counter in order: when a march unit waits for detection
+// (unit_next[1] counts the finished units), every detection unit is with a
+// warp that is running and waits for nothing, so the wait ends, however few of
+// the CTAs fit beside other work on the GPU.
+// Without `detect` (timing a shape) the pass feeds no outlets and latches
+// nothing: it leaves all that the next step reads as it is.  Episodes hold
+// fewer than 2^22 cells, so every moment index fits in 32 bits.
 template <typename T>
 __global__ void __launch_bounds__(32, kMarchWarps)
     pool_dense_kernel(const PoolEpisode *eps, const PoolActive *act, LinkTable lt, uint32_t *owner, uint32_t *unit_next,
@@ -123,16 +130,14 @@ __global__ void __launch_bounds__(32, kMarchWarps)
 {
     __shared__ march2::Ends ends;
     after_predecessor();
+    auto take = [&] { return threadIdx.x == 0 ? atomicAdd(unit_next, 1u) : 0u; };
+    const uint32_t initial = take();
     const int n = (int)act->n;
     if (n == 0) return;
     const uint32_t elements = act->elem_prefix[n], first = detect ? (elements + 3) / 4 : 0u;
     const uint32_t total = first + act->tile_prefix[n];
-    auto take = [&] {
-        uint32_t t = 0;
-        if (threadIdx.x == 0) t = gridDim.x + atomicAdd(unit_next, 1u);
-        return t;
-    };
-    uint32_t t = blockIdx.x;
+    uint32_t t = __shfl_sync(0xffffffffu, initial, 0);
+    march2::Gate gate{unit_next + 1, first, !detect};
     while (t < total) {
         const uint32_t next = take();
         if (t < first) {
@@ -144,14 +149,20 @@ __global__ void __launch_bounds__(32, kMarchWarps)
                                      episode_surface(e), StepScalars{e.cl, e.ct, e.cf},
                                      (long long)(ge - act->elem_prefix[a]), mine < elements, 8,
                                      reinterpret_cast<uint32_t *>(&ends), e.cell_base, owner, s);
+            __syncwarp();
+            if (threadIdx.x == 0) {
+                __threadfence();
+                atomicAdd(unit_next + 1, 1u);
+            }
         } else {
             const int a = owner_of(act->tile_prefix, n, t - first);
             const uint32_t u = t - first - act->tile_prefix[a], W = act->tiles_x[a];
-            const GridArgs<T> g = episode_args<T>(eps[act->slot[a]], parity);
+            GridArgs<T> g = episode_args<T>(eps[act->slot[a]], parity);
+            if (!detect) g.feed = 0;
             const int c = (int)(u / W), w = (int)(u - c * W);
             const int yb = c * rows, ye = min(yb + rows, g.ny);
-            if (g.nx % 2 == 0) march2::run<T, true>(g, w, yb, ye, ends);
-            else march2::run<T, false>(g, w, yb, ye, ends);
+            if (g.nx % 2 == 0) march2::run<T, true>(g, w, yb, ye, ends, gate);
+            else march2::run<T, false>(g, w, yb, ye, ends, gate);
         }
         t = __shfl_sync(0xffffffffu, next, 0);
     }

@@ -114,7 +114,7 @@ __device__ __forceinline__ void dense2d_update_cell(const GridArgs<T> &g, uint32
         encode_store<2, T>(m, planes, idx, g.codec);
     }
     if (bad_state<2>(m)) atomicOr(g.status, kStatusNonFinite);
-    if (f8 & kBitOutletSrc) {
+    if (f8 & g.feed) {
         float ms[6];
         stored_values<2, T>(m, ms, idx, g.codec);
         feed_outlets<2, T>(g, idx, ms, wm);

@@ -359,7 +359,8 @@ template <typename T> constexpr int kThreads3 = D3::kTile + (kRingWarps<T> ? 64 
 // IDX32: every moment, flag and mask index (k * ncell + cell) fits in 32
 // bits, as it does for grids of up to 429 M cells; each access then takes one
 // 32-bit index and one widening multiply-add instead of 64-bit arithmetic.
-template <typename T, bool IDX32>
+// FEED: the pass feeds outlets itself (GridArgs::feed).
+template <typename T, bool IDX32, bool FEED>
 __global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g, const MomentPlanes<T> mp, int zchunk)
 {
     extern __shared__ __align__(128) float smem[];
@@ -595,7 +596,7 @@ __global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g,
                     if constexpr (IDX32) encode_store<3, T>(m, mp.dst, idx, g.codec);
                     else encode_store_strided<3, T>(m, g.dst, (size_t)idx, g.ncell, g.codec);
                     if (bad_state<3>(m)) atomicOr(g.status, kStatusNonFinite);
-                    if (fp & kBitOutletSrc) {
+                    if (FEED && (fp & kBitOutletSrc)) {
                         float ms[10];
                         stored_values<3, T>(m, ms, idx, g.codec);
                         feed_outlets<3, T>(g, idx, ms, wp);
@@ -686,11 +687,11 @@ static int choose_zchunks(int tiles, int nz, int slots)
     return best;
 }
 
-template <typename T, bool IDX32> static cudaError_t launch_as(const GridArgs<T> &g, cudaStream_t s)
+template <typename T, bool IDX32, bool FEED> static cudaError_t launch_as(const GridArgs<T> &g, cudaStream_t s)
 {
     int slots = 0;
     const cudaError_t e =
-        resident_slots(reinterpret_cast<const void *>(dense3d_kernel<T, IDX32>), kThreads3<T>, D3::kSmemBytes, slots);
+        resident_slots(reinterpret_cast<const void *>(dense3d_kernel<T, IDX32, FEED>), kThreads3<T>, D3::kSmemBytes, slots);
     if (e != cudaSuccess) return e;
     int tx = (g.nx + kTX - 1) / kTX, ty = (g.ny + kTY - 1) / kTY;
     int nchunk = choose_zchunks(tx * ty, g.nz, slots);
@@ -701,7 +702,7 @@ template <typename T, bool IDX32> static cudaError_t launch_as(const GridArgs<T>
         mp.src[k] = g.src + (size_t)k * g.ncell;
         mp.dst[k] = g.dst + (size_t)k * g.ncell;
     }
-    dense3d_kernel<T, IDX32><<<grid, kThreads3<T>, D3::kSmemBytes, s>>>(g, mp, zchunk);
+    dense3d_kernel<T, IDX32, FEED><<<grid, kThreads3<T>, D3::kSmemBytes, s>>>(g, mp, zchunk);
     return cudaGetLastError();
 }
 
@@ -710,8 +711,9 @@ template <typename T, bool IDX32> static cudaError_t launch_as(const GridArgs<T>
 template <typename T> cudaError_t launch_dense3d(const GridArgs<T> &g, cudaStream_t s)
 {
     const char *force64 = std::getenv("FFS_DENSE3D_INDEX64");
-    if (10ull * g.ncell <= 0xFFFFFFFFull && !(force64 && force64[0] == '1')) return launch_as<T, true>(g, s);
-    return launch_as<T, false>(g, s);
+    if (10ull * g.ncell <= 0xFFFFFFFFull && !(force64 && force64[0] == '1'))
+        return g.feed ? launch_as<T, true, true>(g, s) : launch_as<T, true, false>(g, s);
+    return g.feed ? launch_as<T, false, true>(g, s) : launch_as<T, false, false>(g, s);
 }
 
 template cudaError_t launch_dense3d<float>(const GridArgs<float> &, cudaStream_t);

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) detect_links3_kernel(GridArgs<T> g, uint3
             const geom::Hit h = geom::isect3_pre(tr, p1, p2);
             if (!h.hit) return;
             const uint32_t cell = (uint32_t)(((long long)k3 * g.ny + j) * g.nx + i);
-            insert_link<Q>(lt, flag_words, cell, ll, geom::link_key(h.depth, (uint32_t)e), g.status);
+            insert_link<3>(g, lt, flag_words, cell, ll, geom::link_key(h.depth, (uint32_t)e));
         };
         const bool queued = hi[0] - lo[0] < 1024 && hi[1] - lo[1] < 1024 && hi[2] - lo[2] < 128;
         int qn = 0;
@@ -297,7 +297,8 @@ __device__ __forceinline__ void finalize_force(const SurfaceArgs &s, long long t
 }
 
 template <int DIM, typename T, bool HALF, bool FOLD>
-__global__ void __launch_bounds__(256, 5) link_cells_kernel(GridArgs<T> g, uint32_t *flag_words, LinkTable lt, SurfaceArgs s,
+__global__ void __launch_bounds__(256, DIM == 2 ? 2 : 5) link_cells_kernel(const __grid_constant__ GridArgs<T> g,
+                                                         uint32_t *flag_words, LinkTable lt, SurfaceArgs s,
                                                          StepScalars sc)
 {
     constexpr int Q = Lattice<DIM>::Q, G = kLinkGroup<DIM>, kPerWarp = 32 / G;
@@ -305,6 +306,7 @@ __global__ void __launch_bounds__(256, 5) link_cells_kernel(GridArgs<T> g, uint3
     const uint32_t group = (threadIdx.x & 31) / G;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     after_predecessor();
+    const uint32_t feeders = g.feeders[0];
     const LinkItems items(lt);
     const uint32_t n = items.n;
     // consecutive cells go to different CTAs: a few cells spread over the SMs
@@ -323,6 +325,8 @@ __global__ void __launch_bounds__(256, 5) link_cells_kernel(GridArgs<T> g, uint3
             set_link_bit(flag_words, cell, false);
         }
     }
+    // the outlets of all other feeders, by the warps without link cells first
+    if (feeders) feed_pass<DIM, T>(g, feeders, flag_words, nwarps - 1 - ((threadIdx.x >> 5) * gridDim.x + blockIdx.x), nwarps);
     if constexpr (!FOLD) return;
     // The CTA that finishes last converts the force sums: every other CTA's
     // atomics are complete and fenced before its count.  No CTA waits for

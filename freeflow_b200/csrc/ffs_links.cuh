@@ -105,7 +105,8 @@ cudaError_t launch_gather_surface(int dim, const float *vpos, const float *vvel,
                                   float *spos, float *svel, float *vforces, uint32_t *status, cudaStream_t st);
 
 template <int DIM>
-cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, int nx, int ny, int nz, cudaStream_t st);
+cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, uint32_t *feeders, uint32_t feeders_cap, int nx, int ny,
+                                 int nz, cudaStream_t st);
 template <int DIM, typename T>
 cudaError_t launch_initialize(const GridArgs<T> &g, T *other, const float *bcvel, cudaStream_t st);
 cudaError_t launch_fill_solid2(uint8_t *flags, int nx, int ny, float cl, const SurfaceArgs &s, cudaStream_t st);

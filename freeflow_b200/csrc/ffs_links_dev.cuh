@@ -15,11 +15,10 @@ __device__ __forceinline__ uint32_t hash_cell(uint32_t c)
     return c;
 }
 
-__device__ __forceinline__ void set_link_bit(uint32_t *flag_words, uint32_t cell, bool on)
+__device__ __forceinline__ uint32_t set_link_bit(uint32_t *flag_words, uint32_t cell, bool on)
 {
     uint32_t bit = (uint32_t)kBitLink << (8 * (cell & 3));
-    if (on) atomicOr(flag_words + (cell >> 2), bit);
-    else atomicAnd(flag_words + (cell >> 2), ~bit);
+    return on ? atomicOr(flag_words + (cell >> 2), bit) : atomicAnd(flag_words + (cell >> 2), ~bit);
 }
 
 // The occupied slots of a table, numbered across its segments: every lane of
@@ -78,11 +77,14 @@ __device__ __forceinline__ void clear_counts(const LinkTable &lt)
 // with owner_id in `owner` when that array is given.  A lane waits for one or
 // two round trips to L2 here (the compare-and-swap, and the list position of a
 // new slot), which is most of a small surface's detection time.
-template <int Q>
-__device__ __forceinline__ void insert_link(const LinkTable &lt, uint32_t *flag_words, uint32_t cell, int l,
-                                            unsigned long long key, uint32_t *status, uint32_t key_base = 0,
+// The claiming thread also marks the outlet nodes the cell feeds, unless the
+// dense pass sees to them (mark_outlets).
+template <int DIM, typename T>
+__device__ __forceinline__ void insert_link(const GridArgs<T> &g, const LinkTable &lt, uint32_t *flag_words, uint32_t cell,
+                                            int l, unsigned long long key, uint32_t key_base = 0,
                                             uint32_t *owner = nullptr, uint32_t owner_id = 0)
 {
+    constexpr int Q = Lattice<DIM>::Q;
     const uint32_t tkey = key_base + cell + 1;
     uint32_t slot = hash_cell(tkey - 1) & (lt.cap - 1);
     for (uint32_t probe = 0; probe < lt.cap; ++probe) {
@@ -93,14 +95,16 @@ __device__ __forceinline__ void insert_link(const LinkTable &lt, uint32_t *flag_
                 const uint32_t seg = slot >> lt.seg_shift;
                 const uint32_t pos = atomicAdd(lt.count + seg * kCountStride, 1u);
                 if (owner) owner[slot] = owner_id;
-                set_link_bit(flag_words, cell, true);
+                const uint32_t was = set_link_bit(flag_words, cell, true) >> (8 * (cell & 3));
                 lt.list[(seg << lt.seg_shift) + pos] = slot;
+                if ((was & kBitOutletSrc) && !g.feed)
+                    mark_outlets<DIM>(flag_words, g.wallmask, g.nx, (long long)g.nx * g.ny, cell);
             }
             return;
         }
         slot = (slot + 1) & (lt.cap - 1);
     }
-    atomicOr(status, kStatusLinkOverflow);
+    atomicOr(g.status, kStatusLinkOverflow);
 }
 
 // D2Q9 link detection of segment e by one warp: every cell of the segment's
@@ -166,7 +170,7 @@ __device__ __forceinline__ void detect_element2_warp(const GridArgs<T> &g, uint3
                                          geom::mul(geom::sub((float)j, (float)dy), cl));
         if (!h.hit) return;
         const uint32_t cell = (uint32_t)((long long)j * g.nx + i);
-        insert_link<Q>(lt, flag_words, cell, ll, geom::link_key(h.depth, (uint32_t)e), g.status, key_base, owner,
+        insert_link<2>(g, lt, flag_words, cell, ll, geom::link_key(h.depth, (uint32_t)e), key_base, owner,
                        owner_id);
     };
     int ci = lane >> 3, cj = 0;
@@ -326,7 +330,7 @@ __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint
                                                      geom::mul(geom::sub((float)j, (float)cy), cl));
                     if (!h.hit) continue;
                     const uint32_t cell = (uint32_t)((long long)j * g.nx + i);
-                    insert_link<Q>(lt, flag_words, cell, l, geom::link_key(h.depth, (uint32_t)e), g.status, key_base, owner,
+                    insert_link<2>(g, lt, flag_words, cell, l, geom::link_key(h.depth, (uint32_t)e), key_base, owner,
                                    owner_id);
                 }
             }
@@ -347,6 +351,7 @@ __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint
         gf.nx = of(g.nx);
         gf.ny = of(g.ny);
         gf.status = of(g.status);
+        gf.wallmask = of(g.wallmask);
         SurfaceArgs sf = s;
         sf.V = of(s.V);
         sf.E = of(s.E);

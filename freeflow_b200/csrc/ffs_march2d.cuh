@@ -235,7 +235,7 @@ __device__ __forceinline__ void encode(const f2 *m, f2 d, uint32_t hash, const C
 template <typename T> __device__ __noinline__ void edge_cell(const GridArgs<T> g, int x, int y)
 {
     const uint32_t idx = (uint32_t)(y * g.nx + x);
-    const uint32_t f8 = g.flags[idx];
+    const uint32_t f8 = __ldcg(reinterpret_cast<const unsigned char *>(g.flags) + idx);
     if (!is_updated(f8 & kTypeMask) || (f8 & kBitLink)) return;
     const bool wx = g.periodic & 1, wy = g.periodic & 2;
     auto population = [&](uint32_t cell, int i) {
@@ -257,35 +257,41 @@ template <typename T> __device__ __noinline__ void edge_cell(const GridArgs<T> g
         [&](int i) { return population(idx, i); });
 }
 
-// Outlets fed by cell p, whose new moments this warp has stored (feed_outlets
-// with one body for the four rules: the code is met cold, at the end of a
-// unit, and four copies of it took longer to fetch than to run).
-template <typename T> __device__ __noinline__ void feed_cell(const GridArgs<T> g, uint32_t p)
-{
-    float ms[6];
-    load_moments<2, T>(ms, g.dst, g.ncell, p, g.codec);
-#pragma unroll 1
-    for (uint32_t word = g.wallmask[p] & outlet_bits_mask<2>(); word; word &= word - 1) {
-        const int r = __ffs(word) - 17; // outlet_bit<2>(r) = 1 << (16 + r)
-        const uint32_t q = (uint32_t)((long long)p + outlet_offset<2>(r, g.nx, 0));
-        const OutletRule rule = outlet_rule<2>(r);
-        const float up = rule.comp == 1 ? ms[1] : ms[2];
-        const bool outward = (rule.sign > 0 && up > 0.0f) || (rule.sign < 0 && up < 0.0f);
-        if constexpr (!StorageTraits<T>::kEncoded) {
-            if (outward) g.dst[(size_t)rule.comp * g.ncell + q] = up;
-            g.dst[(size_t)rule.pcomp * g.ncell + q] = up * up;
-        } else {
-            float mq[6];
-            load_moments<2, T>(mq, g.dst, g.ncell, q, g.codec);
-#pragma unroll
-            for (int k = 1; k < 5; ++k) {
-                if (k == rule.comp && outward) mq[k] = up;
-                if (k == rule.pcomp) mq[k] = up * up;
-            }
-            encode_store_strided<2, T>(mq, g.dst, q, g.ncell, g.codec);
-        }
+// What a unit waits for before it feeds outlets or latches a bad state, both of
+// which must not come from a cell whose links are not known yet: `*done` to
+// reach `want` (the pool's detection units).  Polled by each lane for itself.
+// The wait ends well within a launch (pool_dense_kernel); past its limit
+// (seconds) the status says that the step is invalid.  A warp keeps its gate
+// from unit to unit, open once it was seen open: a look at the counter in every
+// unit with outlets took 4 % of the pool's step.
+// dry: nothing is fed or latched.
+struct Gate {
+    const uint32_t *done;
+    uint32_t want;
+    bool dry;
+    __device__ __forceinline__ void wait(uint32_t *status)
+    {
+        if (want == 0) return;
+        poll(done, want, status);
+        want = 0;
     }
+    static __device__ __noinline__ void poll(const uint32_t *done, uint32_t want, uint32_t *status)
+    {
+        for (uint32_t k = 0; k < (1u << 24); ++k) {
+            uint32_t v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+            if (v >= want) return;
+            __nanosleep(100);
+        }
+        atomicOr(status, kStatusWaitTimeout);
+    }
+};
+template <typename T> __device__ __forceinline__ bool is_link(const GridArgs<T> &g, uint32_t cell)
+{
+    return __ldcg(reinterpret_cast<const unsigned char *>(g.flags) + cell) & kBitLink;
 }
+
+template <typename T> __device__ __noinline__ void feed_outlet_of(const GridArgs<T> g, uint32_t p) { feed_cell<2, T>(g, p, nullptr); }
 
 // Shared memory of a unit's warp: per end, row (yb - 1 + index) and power of
 // c_y, the completed sums that the end column sends in.
@@ -296,7 +302,7 @@ struct Ends {
 // Updates columns 64 w .. 64 w + 63 of rows yb .. ye - 1 (at most kMaxRows).  Every moment
 // index k ncell + cell fits in 32 bits (the caller guarantees it).
 template <typename T, bool VEC>
-__device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye, Ends &ends)
+__device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye, Ends &ends, Gate &gate)
 {
     using P = typename Pair<T>::type;
     const unsigned full = 0xffffffffu;
@@ -310,6 +316,7 @@ __device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye,
     const bool out0 = x < g.nx, out1 = x + 1 < g.nx;
     const bool edge0 = !wx && x == g.nx - 1, edge1 = !wx && x + 1 == g.nx - 1;
     bool edges = false;                 // a Fluid cell on a high face was met
+    uint32_t bad = 0;                   // rows whose cells came out in a bad state: bits 0.. and 16..
     uint32_t feeders0 = 0, feeders1 = 0; // rows (from yb) whose cell feeds an outlet
     const uint32_t fastflags = out0 && out1 && !edge0 && !edge1 ? 0x0101u : 0x10000u; // two plain Fluid cells
 
@@ -492,7 +499,8 @@ __device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye,
         const float inf = __int_as_float(0x7f800000);
         if (!(fminf(ra, rb) > 0.0f && fabsf(sa + sb) < inf)) {
             const bool b0 = !(ra > 0.0f) || !isfinite(sa), b1 = !(rb > 0.0f) || !isfinite(sb);
-            if ((b0 && ((out0 && fast) || st0)) || (b1 && ((out1 && fast) || st1))) atomicOr(g.status, kStatusNonFinite);
+            if (b0 && ((out0 && fast) || st0)) bad |= 1u << (o - yb);
+            if (b1 && ((out1 && fast) || st1)) bad |= 0x10000u << (o - yb);
         }
         if (VEC && fast) {
 #pragma unroll
@@ -563,6 +571,16 @@ __device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye,
         if (r + 1 > ye) break;
         step(r + 1, raw[1], fl[1], wm[0], wm[1]);
     }
+    if (gate.dry) bad = 0, edges = false;
+    if (!g.feed) feeders0 = feeders1 = 0;
+    if (__any_sync(full, edges || (bad | feeders0 | feeders1) != 0)) gate.wait(g.status);
+    for (; bad; bad &= bad - 1) {
+        const int r = __ffs(bad) - 1;
+        if (!is_link(g, (uint32_t)(yb + (r & 15)) * (uint32_t)g.nx + (uint32_t)(x + (r >> 4)))) {
+            atomicOr(g.status, kStatusNonFinite);
+            break;
+        }
+    }
     if (__any_sync(full, (feeders0 | feeders1) != 0)) {
         __syncwarp(); // the feeders' new moments, stored by other lanes
         // Each call is two round trips to L2, so a warp makes as few as it can:
@@ -577,13 +595,13 @@ __device__ __forceinline__ void run(const GridArgs<T> &g, int w, int yb, int ye,
             const uint32_t f0 = __shfl_sync(full, feeders0, from), f1 = __shfl_sync(full, feeders1, from);
             const int r = lane & 15;
             if ((lane < 16 ? f0 : f1) >> r & 1u)
-                feed_cell<T>(g, (uint32_t)(yb + r) * (uint32_t)g.nx + (uint32_t)(kWindow * w + 2 * from + (lane >> 4)));
+                feed_outlet_of<T>(g, (uint32_t)(yb + r) * (uint32_t)g.nx + (uint32_t)(kWindow * w + 2 * from + (lane >> 4)));
         }
         if (!mine) {
             for (uint32_t f = feeders0; f; f &= f - 1)
-                feed_cell<T>(g, (uint32_t)(yb + __ffs(f) - 1) * (uint32_t)g.nx + (uint32_t)x);
+                feed_outlet_of<T>(g, (uint32_t)(yb + __ffs(f) - 1) * (uint32_t)g.nx + (uint32_t)x);
             for (uint32_t f = feeders1; f; f &= f - 1)
-                feed_cell<T>(g, (uint32_t)(yb + __ffs(f) - 1) * (uint32_t)g.nx + (uint32_t)x + 1);
+                feed_outlet_of<T>(g, (uint32_t)(yb + __ffs(f) - 1) * (uint32_t)g.nx + (uint32_t)x + 1);
         }
     }
     if (edges) {

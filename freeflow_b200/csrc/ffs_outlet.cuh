@@ -5,11 +5,12 @@
 // FsiCoupling3D.cu:336-420): an outlet node q copies the normal velocity of its
 // inner neighbour p = q - n (a Fluid node) when that velocity points outward,
 // and sets pi_nn = u_n(p)^2, in place on the freshly written buffer.  Each
-// outlet has exactly one feeder p, and p's new moments are final once p is
-// updated, so the same writes are issued here by the thread that updates p,
-// straight into the buffer being written.  No other node reads q's entries
+// outlet has exactly one feeder p, so the same writes are issued here once p's
+// new moments are final, straight into the buffer being written.  No other node reads q's entries
 // of that buffer during the step, so the result is the reference's.
 #pragma once
+#include <type_traits>
+
 #include "ffs_common.cuh"
 
 namespace fflbm {
@@ -81,6 +82,97 @@ template <int DIM> __host__ __device__ constexpr uint32_t outlet_bits_mask()
 template <int DIM> __host__ __device__ constexpr uint32_t wall_bits_mask()
 {
     return DIM == 2 ? 0x1FEu : 0x07FFFFFEu;
+}
+
+// Who feeds.  Every outlet node has one feeder and is fed once a step, with the
+// feeder's final moments: a feed keeps part of what the node holds, so a feed
+// with a value that is replaced later could not be undone.  The dense pass
+// updates cells beside link detection, and a cell whose links it does not
+// know yet is rewritten by the link-cell kernel.  So:
+//   * a step without a surface: the dense pass feeds (GridArgs::feed);
+//   * a link cell feeds its own outlets (link_cell_update*);
+//   * the other feeders of a step with a surface are fed for by warps of the
+//     link-cell kernel (feed_pass); detection marks the outlet nodes of link
+//     cells for it, because their LINK bits go while it runs (mark_outlets);
+//   * the serving pool's march waits for detection before it feeds
+//     (march2::Gate).
+//
+// Marks the outlet nodes that cell p feeds; p has just been found to have links.
+template <int DIM>
+__device__ __noinline__ void mark_outlets(uint32_t *flag_words, const uint32_t *wallmask, int nx, long long nxy, uint32_t p)
+{
+    const uint32_t word = wallmask[p];
+    for (int r = 0; r < kNumOutletRules<DIM>; ++r) {
+        if (!(word & outlet_bit<DIM>(r))) continue;
+        const uint32_t q = (uint32_t)((long long)p + outlet_offset<DIM>(r, nx, nxy));
+        atomicOr(flag_words + (q >> 2), (uint32_t)kBitOutletSrc << (8 * (q & 3)));
+    }
+}
+
+// Outlets fed by cell p, whose new moments are in g.dst, in one body for all
+// rules: this code is met cold, and a copy per rule took longer to fetch than
+// to run.  Link cells are left out: by their LINK bit, or with flag_words (bits
+// are on their way out) by the marks of their outlet nodes, which are taken off.
+template <int DIM, typename T>
+__device__ __forceinline__ void feed_cell(const GridArgs<T> &g, uint32_t p, uint32_t *flag_words)
+{
+    constexpr int NM = Lattice<DIM>::NM;
+    const long long nxy = (long long)g.nx * g.ny;
+    uint32_t word = g.wallmask[p] & outlet_bits_mask<DIM>();
+    if (!flag_words && (__ldcg(reinterpret_cast<const unsigned char *>(g.flags) + p) & kBitLink)) return;
+#pragma unroll 1
+    for (; word; word &= word - 1) {
+        const int b = __ffs(word) - 1, r = DIM == 2 ? b - 16 : b ? b - 27 : 5; // outlet_bit
+        const uint32_t q = (uint32_t)((long long)p + outlet_offset<DIM>(r, g.nx, nxy));
+        if (flag_words && (g.flags[q] & kBitOutletSrc)) {
+            atomicAnd(flag_words + (q >> 2), ~((uint32_t)kBitOutletSrc << (8 * (q & 3))));
+            continue;
+        }
+        const OutletRule rule = outlet_rule<DIM>(r);
+        float up = StorageTraits<T>::from_vel(g.dst[(size_t)rule.comp * g.ncell + p]);
+        if constexpr (StorageTraits<T>::kEncoded) up *= g.codec.inv_su;
+        const bool outward = (rule.sign > 0 && up > 0.0f) || (rule.sign < 0 && up < 0.0f);
+        if constexpr (!StorageTraits<T>::kEncoded) {
+            if (outward) g.dst[(size_t)rule.comp * g.ncell + q] = up;
+            g.dst[(size_t)rule.pcomp * g.ncell + q] = up * up;
+        } else {
+            float mq[NM];
+            load_moments<DIM, T>(mq, g.dst, g.ncell, q, g.codec);
+#pragma unroll
+            for (int k = 1; k <= 2 * DIM; ++k) {
+                if (k == rule.comp && outward) mq[k] = up;
+                if (k == rule.pcomp) mq[k] = up * up;
+            }
+            encode_store_strided<DIM, T>(mq, g.dst, q, g.ncell, g.codec);
+        }
+    }
+}
+
+// feed_pass for grids with more feeders than their list holds: the feeders are
+// found in the flag bytes, by warps `warp` of `nwarps`.
+template <int DIM, typename T>
+__device__ __noinline__ void feed_scan(const GridArgs<T> &g, uint32_t *flag_words, uint32_t warp, uint32_t nwarps)
+{
+    constexpr uint32_t kFeeder = 0x01010101u * (kBitOutletSrc | kFluid), kSeen = 0x01010101u * (kBitOutletSrc | kTypeMask);
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(g.flags); // the bytes up to a whole word are there, zero
+    const uint32_t n = (g.ncell + 3) / 4;
+    for (uint32_t i = warp * 32 + (threadIdx.x & 31); i < n; i += nwarps * 32)
+        for (uint32_t f = __vcmpeq4(words[i] & kSeen, kFeeder) & 0x01010101u; f; f &= f - 1)
+            feed_cell<DIM, T>(g, 4 * i + (uint32_t)(__ffs(f) - 1) / 8, flag_words);
+}
+
+// Feeds the outlets of the grid's n = g.feeders[0] feeders but the link cells,
+// by warps `warp` of `nwarps`.  The list of feeders was made when the node types were
+// set; finding them in the flag bytes took 1 us of a 17 us step on 800 x 300.
+template <int DIM, typename T>
+__device__ __noinline__ void feed_pass(const GridArgs<T> &g, uint32_t n, uint32_t *flag_words, uint32_t warp, uint32_t nwarps)
+{
+    if (n > g.feeders_cap) {
+        feed_scan<DIM, T>(g, flag_words, warp, nwarps);
+        return;
+    }
+    for (uint32_t i = warp * 32 + (threadIdx.x & 31); i < n; i += nwarps * 32)
+        feed_cell<DIM, T>(g, g.feeders[1 + i], flag_words);
 }
 
 // Called by the thread that has just stored cell p's new moments into g.dst.

@@ -192,7 +192,8 @@ struct ffs_pool {
     PoolOutput *d_out = nullptr, *h_out[2] = {};
     LinkTable lt;
     uint32_t *owner = nullptr;
-    uint32_t *unit_next = nullptr; // next march unit of the dense pass, behind the link counts; zeroed by kinematics
+    uint32_t *unit_next = nullptr; // next unit of the dense pass and its finished detection units, behind the link
+                                   // counts; zeroed by kinematics
     int shape = 1;
     bool act_dirty = true;
     int64_t tuned_cells = 0; // cells of the mix at the last tuning (0: never)
@@ -325,11 +326,12 @@ template <typename T> ffs_status tune_impl(ffs_pool *p)
         p->shape = sh;
         ffs_status r = upload_active(p);
         if (r != FFS_OK) return r;
-        // the dense pass reads the current buffer and writes the other one,
-        // which the next real step overwrites: repeating it changes no state
+        // the dense pass reads the current buffer and writes updated cells of
+        // the other one, which the next real step overwrites; without
+        // detection it leaves outlets and status words alone
         for (int r2 = -1; r2 < 5; ++r2) {
             if (r2 == 0) POOL_CK(cudaEventRecord(p->ev0, p->st));
-            POOL_CK(cudaMemsetAsync(p->unit_next, 0, sizeof(uint32_t), p->st));
+            POOL_CK(cudaMemsetAsync(p->unit_next, 0, 2 * sizeof(uint32_t), p->st));
             POOL_CK((launch_pool_dense<T>(p->d_eps, p->d_act, p->lt, p->owner, p->unit_next, false, p->parity, sh,
                                           p->grid_dense, p->st)));
         }
@@ -464,11 +466,11 @@ ffs_status ffs_pool_create(const ffs_pool_desc *desc, ffs_pool **out)
     if ((e = cudaMalloc(&p->lt.keys, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link keys");
     if ((e = cudaMalloc(&p->lt.links, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "links");
     if ((e = cudaMalloc(&p->lt.list, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link list");
-    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t) * (kCountWords + 1))) != cudaSuccess) return bail(e, "link count");
+    if ((e = cudaMalloc(&p->lt.count, sizeof(uint32_t) * (kCountWords + 2))) != cudaSuccess) return bail(e, "link count");
     if ((e = cudaMalloc(&p->owner, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "link owner");
     if ((e = cudaMemset(p->lt.keys, 0, sizeof(uint32_t) * cap)) != cudaSuccess) return bail(e, "memset");
     if ((e = cudaMemset(p->lt.links, 0xFF, sizeof(unsigned long long) * cap * 9)) != cudaSuccess) return bail(e, "memset");
-    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t) * (kCountWords + 1))) != cudaSuccess) return bail(e, "memset");
+    if ((e = cudaMemset(p->lt.count, 0, sizeof(uint32_t) * (kCountWords + 2))) != cudaSuccess) return bail(e, "memset");
     p->unit_next = p->lt.count + kCountWords;
     p->lt.acc = nullptr; // per-episode accumulators live in the arena
     p->lt.acc_cap = 0;
@@ -633,7 +635,7 @@ ffs_status ffs_pool_admit(ffs_pool *p, const ffs_episode_desc *ep, int *slot_out
     zero(E.sums, sizeof(double) * 4);
     cp(p->d_eps + si, &E, sizeof(PoolEpisode));
     if (e != cudaSuccess) return undo(fail(FFS_ERR_CUDA, std::string("admission upload: ") + cudaGetErrorString(e)));
-    if ((e = launch_prepare_flags<2>(E.flags, E.wallmask, d.nx, d.ny, 1, st)) != cudaSuccess)
+    if ((e = launch_prepare_flags<2>(E.flags, E.wallmask, nullptr, 0u, d.nx, d.ny, 1, st)) != cudaSuccess)
         return undo(fail(FFS_ERR_CUDA, std::string("prepare flags: ") + cudaGetErrorString(e)));
     switch (p->d.storage) {
     case FFS_STORAGE_F32: r = init_episode<float>(p, s, d.boundary_velocities); break;

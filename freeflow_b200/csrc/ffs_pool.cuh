@@ -127,6 +127,9 @@ template <typename T> __device__ __forceinline__ GridArgs<T> episode_args(const 
     g.periodic = 0;
     g.half_pops = 0;
     g.wall_stream = 0;
+    g.feed = kBitOutletSrc;
+    g.feeders = nullptr;
+    g.feeders_cap = 0;
     g.omega = e.omega;
     g.codec = e.codec;
     g.src = static_cast<const T *>(e.mom[parity]);
