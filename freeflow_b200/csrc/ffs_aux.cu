@@ -26,8 +26,8 @@ template <int DIM> __device__ __forceinline__ void dir3(int i, int &cx, int &cy,
 // pool's grids).  Node types are static between flag uploads, so this runs
 // once per upload instead of every step.
 template <int DIM>
-__global__ void prepare_flags_kernel(uint8_t *flags, uint32_t *wallmask, uint32_t *feeders, uint32_t feeders_cap, int nx,
-                                     int ny, int nz)
+__global__ void prepare_flags_kernel(uint8_t *flags, uint32_t *wallmask, uint2 *feeders, uint32_t *feeders_n,
+                                     uint32_t feeders_cap, int nx, int ny, int nz)
 {
     constexpr int Q = Lattice<DIM>::Q;
     const long long nxy = (long long)nx * ny, n = nxy * nz;
@@ -54,8 +54,8 @@ __global__ void prepare_flags_kernel(uint8_t *flags, uint32_t *wallmask, uint32_
             }
         }
         if (feeders && (bits & kBitOutletSrc)) {
-            const uint32_t at = atomicAdd(feeders, 1u);
-            if (at < feeders_cap) feeders[1 + at] = (uint32_t)c;
+            const uint32_t at = atomicAdd(feeders_n, 1u);
+            if (at < feeders_cap) feeders[at] = make_uint2((uint32_t)c, mask);
         }
         wallmask[c] = mask;
         flags[c] = bits; // neighbours only read the type bits, which do not change
@@ -63,16 +63,16 @@ __global__ void prepare_flags_kernel(uint8_t *flags, uint32_t *wallmask, uint32_
 }
 
 template <int DIM>
-cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, uint32_t *feeders, uint32_t feeders_cap, int nx, int ny,
-                                 int nz, cudaStream_t st)
+cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, uint2 *feeders, uint32_t *feeders_n, uint32_t feeders_cap,
+                                 int nx, int ny, int nz, cudaStream_t st)
 {
     long long n = (long long)nx * ny * nz;
     int grid = (int)std::min<long long>((n + 255) / 256, (long long)device_sms() * 16);
-    prepare_flags_kernel<DIM><<<grid, 256, 0, st>>>(flags, wallmask, feeders, feeders_cap, nx, ny, nz);
+    prepare_flags_kernel<DIM><<<grid, 256, 0, st>>>(flags, wallmask, feeders, feeders_n, feeders_cap, nx, ny, nz);
     return cudaGetLastError();
 }
-template cudaError_t launch_prepare_flags<2>(uint8_t *, uint32_t *, uint32_t *, uint32_t, int, int, int, cudaStream_t);
-template cudaError_t launch_prepare_flags<3>(uint8_t *, uint32_t *, uint32_t *, uint32_t, int, int, int, cudaStream_t);
+template cudaError_t launch_prepare_flags<2>(uint8_t *, uint32_t *, uint2 *, uint32_t *, uint32_t, int, int, int, cudaStream_t);
+template cudaError_t launch_prepare_flags<3>(uint8_t *, uint32_t *, uint2 *, uint32_t *, uint32_t, int, int, int, cudaStream_t);
 
 // initialize_state_kernel_2d/3d (LbmInitializer2D.cu:32-95,
 // LbmInitializer3D.cu:33-113): rho = 1, u set on inlet nodes from the

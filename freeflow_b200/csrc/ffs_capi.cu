@@ -43,7 +43,7 @@ struct ffs_lbm {
     Codec codec{};
     LinkTable lt;
     float *staging = nullptr; // ncell * NM floats, allocated on first host transfer
-    uint32_t *feeders = nullptr;   // [1 + feeders_cap] cells that feed outlets (GridArgs::feeders)
+    uint2 *feeders = nullptr;      // [feeders_cap] cells that feed outlets, and behind them their number (GridArgs)
     uint32_t *fill_bits = nullptr; // D3Q27 solid fill: one parity bit per cell, zero between calls
     // link detection runs on `side` while the dense pass runs on the caller's
     // stream; fork/join order them
@@ -114,6 +114,7 @@ template <typename T> GridArgs<T> args(ffs_lbm *h)
     g.feed = kBitOutletSrc;
     g.feeders = h->feeders;
     g.feeders_cap = feeders_cap(h->dim, h->d.nx, h->d.ny, h->d.nz);
+    g.feeders_n = reinterpret_cast<const uint32_t *>(h->feeders + g.feeders_cap);
     g.omega = h->omega;
     g.codec = h->codec;
     g.src = static_cast<const T *>(h->mom[h->cur]);
@@ -130,6 +131,11 @@ void free_links(LinkTable &lt)
     lt = LinkTable{};
 }
 
+// One claim counter or kSegments of them (LinkTable).  The segments cost a small
+// surface 0.5 us a step (64 lines to read before the first link cell is known);
+// claims in one counter serialise, at about 1 ns each.
+uint32_t claim_segments(int dim, uint32_t cap) { return dim == 2 && cap <= kOneCounterCap ? 31u : segment_shift(cap); }
+
 ffs_status ensure_links(ffs_lbm *h, int64_t max_vertices, int64_t max_link_cells)
 {
     LinkTable &lt = h->lt;
@@ -144,7 +150,7 @@ ffs_status ensure_links(ffs_lbm *h, int64_t max_vertices, int64_t max_link_cells
         FFS_CK(cudaMemset(lt.keys, 0, sizeof(uint32_t) * want_cap));
         FFS_CK(cudaMemset(lt.links, 0xFF, sizeof(unsigned long long) * (size_t)want_cap * h->Q));
         lt.cap = want_cap;
-        lt.seg_shift = segment_shift(want_cap);
+        lt.seg_shift = claim_segments(h->dim, want_cap);
     }
     if (!lt.count) {
         // the lists' counts and the finished-CTA count of link_cells_kernel
@@ -357,9 +363,10 @@ int which_index(const ffs_lbm *h, int which)
 ffs_status prepare_flags(ffs_lbm *h, cudaStream_t st)
 {
     const uint32_t cap = feeders_cap(h->dim, h->d.nx, h->d.ny, h->d.nz);
-    FFS_CK(cudaMemsetAsync(h->feeders, 0, sizeof(uint32_t), st));
-    if (h->dim == 2) FFS_CK(launch_prepare_flags<2>(h->flags, h->wallmask, h->feeders, cap, h->d.nx, h->d.ny, 1, st));
-    else FFS_CK(launch_prepare_flags<3>(h->flags, h->wallmask, h->feeders, cap, h->d.nx, h->d.ny, h->d.nz, st));
+    uint32_t *n = reinterpret_cast<uint32_t *>(h->feeders + cap);
+    FFS_CK(cudaMemsetAsync(n, 0, sizeof(uint32_t), st));
+    if (h->dim == 2) FFS_CK(launch_prepare_flags<2>(h->flags, h->wallmask, h->feeders, n, cap, h->d.nx, h->d.ny, 1, st));
+    else FFS_CK(launch_prepare_flags<3>(h->flags, h->wallmask, h->feeders, n, cap, h->d.nx, h->d.ny, h->d.nz, st));
     return FFS_OK;
 }
 
@@ -440,7 +447,7 @@ ffs_status ffs_lbm_create(const ffs_lbm_desc *desc, ffs_lbm **out)
     const size_t fbytes = ((size_t)ncell + 3) & ~(size_t)3;
     if ((e = cudaMalloc(&h->flags, fbytes)) != cudaSuccess) return bail(e, "flags");
     if ((e = cudaMalloc(&h->wallmask, sizeof(uint32_t) * (size_t)ncell)) != cudaSuccess) return bail(e, "wallmask");
-    if ((e = cudaMalloc(&h->feeders, sizeof(uint32_t) * (1 + (size_t)feeders_cap(d.dim, d.nx, d.ny, nz)))) != cudaSuccess)
+    if ((e = cudaMalloc(&h->feeders, sizeof(uint2) * (1 + (size_t)feeders_cap(d.dim, d.nx, d.ny, nz)))) != cudaSuccess)
         return bail(e, "feeders");
     if ((e = cudaMalloc(&h->status, sizeof(uint32_t))) != cudaSuccess) return bail(e, "status");
     if ((e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");

@@ -476,7 +476,8 @@ template <typename T> struct GridArgs {
     T *dst;
     const uint8_t *flags;
     const uint32_t *wallmask; // per-cell bounce-back direction mask (read only for near-wall cells)
-    const uint32_t *feeders; // the number of cells that feed outlets, then up to feeders_cap of them (single grids)
+    const uint2 *feeders;    // up to feeders_cap cells that feed outlets, with their mask words (single grids)
+    const uint32_t *feeders_n; // how many there are
     uint32_t feeders_cap;
     uint32_t *status;
 };

@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(256, DIM == 2 ? 2 : 5) link_cells_kernel(const
     const int lane = threadIdx.x & (G - 1);
     const uint32_t group = (threadIdx.x & 31) / G;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t feeders = *g.feeders_n; // made when the node types were set, long before the dense pass
     after_predecessor();
-    const uint32_t feeders = g.feeders[0];
     const LinkItems items(lt);
     const uint32_t n = items.n;
     // consecutive cells go to different CTAs: a few cells spread over the SMs

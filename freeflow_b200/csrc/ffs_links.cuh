@@ -17,6 +17,7 @@ namespace fflbm {
 // visits to the empty state, so the table is clean again at the end of the
 // step without touching unused slots.
 constexpr uint32_t kSegments = 64, kCountStride = 32;
+constexpr uint32_t kOneCounterCap = 1u << 15; // 2D tables of at most this many slots keep one counter
 constexpr size_t kCountWords = (size_t)kSegments * kCountStride;
 struct LinkTable {
     uint32_t cap = 0;                  // power of two (0: not allocated)
@@ -105,8 +106,8 @@ cudaError_t launch_gather_surface(int dim, const float *vpos, const float *vvel,
                                   float *spos, float *svel, float *vforces, uint32_t *status, cudaStream_t st);
 
 template <int DIM>
-cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, uint32_t *feeders, uint32_t feeders_cap, int nx, int ny,
-                                 int nz, cudaStream_t st);
+cudaError_t launch_prepare_flags(uint8_t *flags, uint32_t *wallmask, uint2 *feeders, uint32_t *feeders_n, uint32_t feeders_cap,
+                                 int nx, int ny, int nz, cudaStream_t st);
 template <int DIM, typename T>
 cudaError_t launch_initialize(const GridArgs<T> &g, T *other, const float *bcvel, cudaStream_t st);
 cudaError_t launch_fill_solid2(uint8_t *flags, int nx, int ny, float cl, const SurfaceArgs &s, cudaStream_t st);

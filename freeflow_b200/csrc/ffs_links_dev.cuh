@@ -15,10 +15,11 @@ __device__ __forceinline__ uint32_t hash_cell(uint32_t c)
     return c;
 }
 
-__device__ __forceinline__ uint32_t set_link_bit(uint32_t *flag_words, uint32_t cell, bool on)
+__device__ __forceinline__ void set_link_bit(uint32_t *flag_words, uint32_t cell, bool on)
 {
     uint32_t bit = (uint32_t)kBitLink << (8 * (cell & 3));
-    return on ? atomicOr(flag_words + (cell >> 2), bit) : atomicAnd(flag_words + (cell >> 2), ~bit);
+    if (on) atomicOr(flag_words + (cell >> 2), bit);
+    else atomicAnd(flag_words + (cell >> 2), ~bit);
 }
 
 // The occupied slots of a table, numbered across its segments: every lane of
@@ -87,6 +88,8 @@ __device__ __forceinline__ void insert_link(const GridArgs<T> &g, const LinkTabl
     constexpr int Q = Lattice<DIM>::Q;
     const uint32_t tkey = key_base + cell + 1;
     uint32_t slot = hash_cell(tkey - 1) & (lt.cap - 1);
+    // (fetched beside the compare-and-swap)
+    const bool feeds = !g.feed && (reinterpret_cast<const uint8_t *>(flag_words)[cell] & kBitOutletSrc);
     for (uint32_t probe = 0; probe < lt.cap; ++probe) {
         const uint32_t old = atomicCAS(lt.keys + slot, 0u, tkey);
         if (old == 0u || old == tkey) {
@@ -95,10 +98,9 @@ __device__ __forceinline__ void insert_link(const GridArgs<T> &g, const LinkTabl
                 const uint32_t seg = slot >> lt.seg_shift;
                 const uint32_t pos = atomicAdd(lt.count + seg * kCountStride, 1u);
                 if (owner) owner[slot] = owner_id;
-                const uint32_t was = set_link_bit(flag_words, cell, true) >> (8 * (cell & 3));
+                set_link_bit(flag_words, cell, true);
                 lt.list[(seg << lt.seg_shift) + pos] = slot;
-                if ((was & kBitOutletSrc) && !g.feed)
-                    mark_outlets<DIM>(flag_words, g.wallmask, g.nx, (long long)g.nx * g.ny, cell);
+                if (feeds) mark_outlets<DIM>(flag_words, g.wallmask, g.nx, (long long)g.nx * g.ny, cell);
             }
             return;
         }

@@ -1,5 +1,6 @@
-// Row-marching body of the fused D2Q9 update, one warp per unit, shared by the
-// single-grid kernel (ffs_dense2d.cu) and the serving pool's (ffs_batch2d.cu).
+// Row-marching body of the fused D2Q9 update, one warp per unit, for the serving
+// pool and large single grids, and the cell update it shares with the tiles of
+// small ones (ffs_dense2d.cu).
 //
 // Reference: mrDeformableSolver2DKernel_Shrd (src/core/FsiCoupling2D.cu:82-255).
 //
@@ -14,8 +15,9 @@
 // by the same shuffles.
 //
 // What bounds it: instruction issue, then HBM.  The tile-and-strip kernels it
-// replaces staged populations in shared memory and spent about 347 thread
-// instructions per cell; the packed march needs about a third of that.
+// replaced in the pool staged populations in shared memory and spent about 347
+// thread instructions per cell; the packed march takes 189 (FP16 serving mix,
+// 14 rows, with detection).
 //
 // Bounce-back: a wall or solid cell is reconstructed from a zero state, so
 // whatever a neighbour pulls from it adds nothing, and a cell next to a wall
@@ -160,36 +162,39 @@ template <typename V> struct Rows {
     }
 };
 
-// collide2 on a pair of cells from the sums S of F': the raw moments are
+// collide2 from the sums S of F', of one cell or a pair: the raw moments are
 // {1 + W0 S0, W0/4 S1, W0/4 S2, 1/3 + W0/4 S3, 1/3 + W0/4 S4, W0/16 S5} with
 // W0 = 4/9 (the lattice weights are W0 times powers of 1/4).  The velocity
 // comes out in its stored scale, u * su (su a power of two, isu2 = su^-2).
-// 1 / rho is the hardware approximation refined by one Newton step, as
-// recip().  d receives rho - 1.
+// d receives rho - 1.
 constexpr float kW0 = wgt2(1, 1);
-__device__ __forceinline__ void collide(const f2 *S, float omega, float su, float isu2, f2 *m, f2 &d)
+__device__ __forceinline__ float vrecip(float r) { return recip(r); }
+__device__ __forceinline__ f2 vrecip(f2 r)
 {
-    float s0, s1;
-    f2split(S[0], s0, s1);
-    const float r0 = fmaf(kW0, s0, 1.0f), r1 = fmaf(kW0, s1, 1.0f);
-    d = f2make(kW0 * s0, kW0 * s1);
-    const float a0 = rcp_approx(r0), a1 = rcp_approx(r1);
-    const float i0 = a0 * fmaf(-r0, a0, 2.0f), i1 = a1 * fmaf(-r1, a1, 2.0f);
-    const f2 wr = f2make(0.25f * kW0 * i0, 0.25f * kW0 * i1); // W0 / (4 rho)
-    const f2 wu = wr * f2splat(su);
-    const f2 ux = S[1] * wu, uy = S[2] * wu; // u * su
-    const f2 k = wr * f2splat(0.5f * (1.0f - omega));
-    const f2 ux2 = ux * ux;
-    const f2 sum = vfma(uy, uy, ux2), dif = vfma(f2splat(-1.0f) * uy, uy, ux2);
+    float r0, r1;
+    f2split(r, r0, r1);
+    return f2make(recip(r0), recip(r1));
+}
+template <typename V> __device__ __forceinline__ void collide(const V *S, float omega, float su, float isu2, V *m, V &d)
+{
+    auto k = [](float a) { return vconst<V>(a); };
+    const V r = vfma(k(kW0), S[0], k(1.0f));
+    d = k(kW0) * S[0];
+    const V wr = k(0.25f * kW0) * vrecip(r); // W0 / (4 rho)
+    const V wu = wr * k(su);
+    const V ux = S[1] * wu, uy = S[2] * wu; // u * su
+    const V kr = wr * k(0.5f * (1.0f - omega));
+    const V ux2 = ux * ux;
+    const V sum = vfma(uy, uy, ux2), dif = vfma(k(-1.0f) * uy, uy, ux2);
     // half the difference of the normal stresses, relaxed
-    const f2 n = vfma(S[3] - S[4], k, f2splat(0.5f * omega * isu2) * dif);
-    const f2 half_u2 = f2splat(0.5f * isu2) * sum;
-    m[0] = f2make(r0, r1);
+    const V n = vfma(S[3] - S[4], kr, k(0.5f * omega * isu2) * dif);
+    const V half_u2 = k(0.5f * isu2) * sum;
+    m[0] = r;
     m[1] = ux;
     m[2] = uy;
     m[3] = half_u2 + n;
     m[4] = half_u2 - n;
-    m[5] = vfma(S[5], f2splat(0.5f) * k, f2splat(omega * isu2) * (ux * uy));
+    m[5] = vfma(S[5], k(0.5f) * kr, k(omega * isu2) * (ux * uy));
 }
 
 // Stored form of a pair (encode_values of both cells; d = rho - 1, hash the
@@ -230,31 +235,125 @@ __device__ __forceinline__ void encode(const f2 *m, f2 d, uint32_t hash, const C
     }
 }
 
+// The same of one cell.
+template <typename T>
+__device__ __forceinline__ void encode(const float *m, float d, uint32_t hash, const Codec &c, T *out)
+{
+    if constexpr (!StorageTraits<T>::kEncoded) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) out[k] = m[k];
+    } else {
+        using Tr = StorageTraits<T>;
+        const uint32_t u = half2_sr(m[1], m[2], mix32(hash ^ __float_as_uint(m[0])));
+        float sx, sy;
+        f2split(halves(u), sx, sy);
+        const float isu2 = -(c.inv_su * c.inv_su), nx = isu2 * sx, ny = isu2 * sy;
+        out[0] = Tr::to(d);
+        out[1] = Tr::to_vel(sx); // binary16 values: exact
+        out[2] = Tr::to_vel(sy);
+        out[3] = Tr::to(fmaf(nx, sx, m[3]) * c.sp);
+        out[4] = Tr::to(fmaf(ny, sy, m[4]) * c.sp);
+        out[5] = Tr::to(fmaf(nx, sy, m[5]) * c.sp);
+    }
+}
+
+// Update of one cell from populations F' given one by one: pull(kx, ky) of the
+// cell that c = (kx - 1, ky - 1) comes from, own(kx, ky) of the cell itself (kx
+// and ky as Rows).  A direction whose wall bit is set sends F = 0 and the cell
+// adds its own reflected population.  wm: the mask word of a cell near walls or
+// feeding outlets.  The operations and their order are run's.
+template <typename T, typename Pull, typename Own>
+__device__ __forceinline__ void update_cell(const GridArgs<T> &g, uint32_t idx, uint32_t f8, uint32_t wm, Pull &&pull, Own &&own)
+{
+    const uint32_t walls = f8 & kBitNearWall ? wm & wall_bits_mask<2>() : 0u;
+    float p[3][3];
+#pragma unroll
+    for (int ky = 0; ky < 3; ++ky)
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) p[ky][kx] = pull(kx, ky);
+    if (walls) {
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky)
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx)
+                if (walls >> dir_index<2>(kx, ky, 1) & 1u) p[ky][kx] = -1.0f;
+    }
+    float Y0[3], Y1[3], Y2[3], S[6];
+#pragma unroll
+    for (int kx = 0; kx < 3; ++kx) {
+        const float A = p[2][kx], C = p[0][kx];
+        Y0[kx] = fmaf(0.25f, C, fmaf(0.25f, A, p[1][kx]));
+        Y1[kx] = A - C;
+        Y2[kx] = A + C;
+    }
+    S[3] = Y0[2] + Y0[0];
+    S[0] = fmaf(0.25f, S[3], Y0[1]);
+    S[1] = Y0[2] - Y0[0];
+    S[2] = fmaf(0.25f, Y1[2] + Y1[0], Y1[1]);
+    S[4] = fmaf(0.25f, Y2[2] + Y2[0], Y2[1]);
+    S[5] = Y1[2] - Y1[0];
+    if (walls) {
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky)
+#pragma unroll
+            for (int kx = 0; kx < 3; ++kx) {
+                if (kx == 1 && ky == 1) continue;
+                const int cx = 1 - kx, cy = 1 - ky;
+                const float w = (cx != 0 && cy != 0) ? 0.0625f : 0.25f; // the weight over W0
+                const float t = walls >> dir_index<2>(2 - kx, 2 - ky, 1) & 1u ? 1.0f + own(kx, ky) : 0.0f;
+                const float t4 = 4.0f * w * t, t16 = 16.0f * w * t;
+                S[0] = fmaf(w, t, S[0]);
+                if (cx) S[1] = cx > 0 ? S[1] + t4 : S[1] - t4;
+                if (cy) S[2] = cy > 0 ? S[2] + t4 : S[2] - t4;
+                if (cx) S[3] = S[3] + t4;
+                if (cy) S[4] = S[4] + t4;
+                if (cx && cy) S[5] = cx * cy > 0 ? S[5] + t16 : S[5] - t16;
+            }
+    }
+    float m[6], d;
+    T e[6];
+    constexpr bool enc = StorageTraits<T>::kEncoded;
+    collide<float>(S, g.omega, enc ? g.codec.su : 1.0f, enc ? g.codec.inv_su * g.codec.inv_su : 1.0f, m, d);
+    encode<T>(m, d, idx * kGolden, g.codec, e);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) g.dst[idx + (uint32_t)k * g.ncell] = e[k];
+    if (bad_state<2>(m)) atomicOr(g.status, kStatusNonFinite);
+    if (f8 & g.feed) {
+        float ms[6] = {};
+#pragma unroll
+        for (int k = 1; k < 3; ++k) ms[k] = StorageTraits<T>::from_vel(e[k]) * (enc ? g.codec.inv_su : 1.0f);
+        feed_outlets<2, T>(g, idx, ms, wm);
+    }
+}
+
+// F' of one cell with c = (kx - 1, ky - 1)
+template <typename T> __device__ __forceinline__ float population(const GridArgs<T> &g, uint32_t cell, int kx, int ky)
+{
+    float m[6], d, F[3];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) m[k] = from_storage<2, T>(k, g.src[cell + (uint32_t)k * g.ncell]);
+    decode_values<T>(g.codec, m, d);
+    const Rows<float> rows(m, d);
+    if (ky == 0) rows.template row<0>(F);
+    else if (ky == 1) rows.template row<1>(F);
+    else rows.template row<2>(F);
+    return fmaxf(F[kx], -1.0f);
+}
+
 // Update of a Fluid cell on the high face of a non-periodic axis, gathering
-// each of its populations from its halo source (dense2d_update_cell).
+// each of its populations from its halo source.
 template <typename T> __device__ __noinline__ void edge_cell(const GridArgs<T> g, int x, int y)
 {
     const uint32_t idx = (uint32_t)(y * g.nx + x);
     const uint32_t f8 = __ldcg(reinterpret_cast<const unsigned char *>(g.flags) + idx);
     if (!is_updated(f8 & kTypeMask) || (f8 & kBitLink)) return;
     const bool wx = g.periodic & 1, wy = g.periodic & 2;
-    auto population = [&](uint32_t cell, int i) {
-        int cx, cy, cz;
-        dir_vec<2>(i, cx, cy, cz);
-        float m[6];
-        load_moments<2, T>(m, g.src, g.ncell, cell, g.codec);
-        Coef<2> cf;
-        cf.make(m);
-        return cf.population(cx, cy, cz);
-    };
-    dense2d_update_cell<T, true>(
-        g, idx, f8,
-        [&](int i) {
-            int cx, cy, cz;
-            dir_vec<2>(i, cx, cy, cz);
-            return population((uint32_t)(halo_index(y - cy, g.ny, wy) * g.nx + halo_index(x - cx, g.nx, wx)), i);
+    update_cell<T>(
+        g, idx, f8, g.wallmask[idx],
+        [&](int kx, int ky) {
+            return population(g, (uint32_t)(halo_index(y + 1 - ky, g.ny, wy) * g.nx + halo_index(x + 1 - kx, g.nx, wx)), kx, ky);
         },
-        [&](int i) { return population(idx, i); });
+        [&](int kx, int ky) { return population(g, idx, kx, ky); });
 }
 
 // What a unit waits for before it feeds outlets or latches a bad state, both of
@@ -291,7 +390,7 @@ template <typename T> __device__ __forceinline__ bool is_link(const GridArgs<T> 
     return __ldcg(reinterpret_cast<const unsigned char *>(g.flags) + cell) & kBitLink;
 }
 
-template <typename T> __device__ __noinline__ void feed_outlet_of(const GridArgs<T> g, uint32_t p) { feed_cell<2, T>(g, p, nullptr); }
+template <typename T> __device__ __noinline__ void feed_outlet_of(const GridArgs<T> g, uint32_t p) { feed_cell<2, T>(g, p, g.wallmask[p], nullptr); }
 
 // Shared memory of a unit's warp: per end, row (yb - 1 + index) and power of
 // c_y, the completed sums that the end column sends in.

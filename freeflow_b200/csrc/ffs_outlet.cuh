@@ -109,35 +109,37 @@ __device__ __noinline__ void mark_outlets(uint32_t *flag_words, const uint32_t *
     }
 }
 
-// Outlets fed by cell p, whose new moments are in g.dst, in one body for all
+// Outlets fed by cell p (mask word `word`), whose new moments are in g.dst, in one body for all
 // rules: this code is met cold, and a copy per rule took longer to fetch than
 // to run.  Link cells are left out: by their LINK bit, or with flag_words (bits
 // are on their way out) by the marks of their outlet nodes, which are taken off.
 template <int DIM, typename T>
-__device__ __forceinline__ void feed_cell(const GridArgs<T> &g, uint32_t p, uint32_t *flag_words)
+__device__ __forceinline__ void feed_cell(const GridArgs<T> &g, uint32_t p, uint32_t word, uint32_t *flag_words)
 {
     constexpr int NM = Lattice<DIM>::NM;
     const long long nxy = (long long)g.nx * g.ny;
-    uint32_t word = g.wallmask[p] & outlet_bits_mask<DIM>();
+    word &= outlet_bits_mask<DIM>();
     if (!flag_words && (__ldcg(reinterpret_cast<const unsigned char *>(g.flags) + p) & kBitLink)) return;
 #pragma unroll 1
     for (; word; word &= word - 1) {
         const int b = __ffs(word) - 1, r = DIM == 2 ? b - 16 : b ? b - 27 : 5; // outlet_bit
         const uint32_t q = (uint32_t)((long long)p + outlet_offset<DIM>(r, g.nx, nxy));
-        if (flag_words && (g.flags[q] & kBitOutletSrc)) {
-            atomicAnd(flag_words + (q >> 2), ~((uint32_t)kBitOutletSrc << (8 * (q & 3))));
-            continue;
-        }
+        // all loads before any is tested
+        const uint32_t fq = flag_words ? g.flags[q] : 0u;
         const OutletRule rule = outlet_rule<DIM>(r);
         float up = StorageTraits<T>::from_vel(g.dst[(size_t)rule.comp * g.ncell + p]);
         if constexpr (StorageTraits<T>::kEncoded) up *= g.codec.inv_su;
+        float mq[NM];
+        if constexpr (StorageTraits<T>::kEncoded) load_moments<DIM, T>(mq, g.dst, g.ncell, q, g.codec);
+        if (fq & kBitOutletSrc) {
+            atomicAnd(flag_words + (q >> 2), ~((uint32_t)kBitOutletSrc << (8 * (q & 3))));
+            continue;
+        }
         const bool outward = (rule.sign > 0 && up > 0.0f) || (rule.sign < 0 && up < 0.0f);
         if constexpr (!StorageTraits<T>::kEncoded) {
             if (outward) g.dst[(size_t)rule.comp * g.ncell + q] = up;
             g.dst[(size_t)rule.pcomp * g.ncell + q] = up * up;
         } else {
-            float mq[NM];
-            load_moments<DIM, T>(mq, g.dst, g.ncell, q, g.codec);
 #pragma unroll
             for (int k = 1; k <= 2 * DIM; ++k) {
                 if (k == rule.comp && outward) mq[k] = up;
@@ -157,11 +159,13 @@ __device__ __noinline__ void feed_scan(const GridArgs<T> &g, uint32_t *flag_word
     const uint32_t *words = reinterpret_cast<const uint32_t *>(g.flags); // the bytes up to a whole word are there, zero
     const uint32_t n = (g.ncell + 3) / 4;
     for (uint32_t i = warp * 32 + (threadIdx.x & 31); i < n; i += nwarps * 32)
-        for (uint32_t f = __vcmpeq4(words[i] & kSeen, kFeeder) & 0x01010101u; f; f &= f - 1)
-            feed_cell<DIM, T>(g, 4 * i + (uint32_t)(__ffs(f) - 1) / 8, flag_words);
+        for (uint32_t f = __vcmpeq4(words[i] & kSeen, kFeeder) & 0x01010101u; f; f &= f - 1) {
+            const uint32_t p = 4 * i + (uint32_t)(__ffs(f) - 1) / 8;
+            feed_cell<DIM, T>(g, p, g.wallmask[p], flag_words);
+        }
 }
 
-// Feeds the outlets of the grid's n = g.feeders[0] feeders but the link cells,
+// Feeds the outlets of the grid's n = *g.feeders_n feeders but the link cells,
 // by warps `warp` of `nwarps`.  The list of feeders was made when the node types were
 // set; finding them in the flag bytes took 1 us of a 17 us step on 800 x 300.
 template <int DIM, typename T>
@@ -171,8 +175,10 @@ __device__ __noinline__ void feed_pass(const GridArgs<T> &g, uint32_t n, uint32_
         feed_scan<DIM, T>(g, flag_words, warp, nwarps);
         return;
     }
-    for (uint32_t i = warp * 32 + (threadIdx.x & 31); i < n; i += nwarps * 32)
-        feed_cell<DIM, T>(g, g.feeders[1 + i], flag_words);
+    for (uint32_t i = warp * 32 + (threadIdx.x & 31); i < n; i += nwarps * 32) {
+        const uint2 f = g.feeders[i];
+        feed_cell<DIM, T>(g, f.x, f.y, flag_words);
+    }
 }
 
 // Called by the thread that has just stored cell p's new moments into g.dst.

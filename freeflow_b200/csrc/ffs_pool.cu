@@ -635,7 +635,7 @@ ffs_status ffs_pool_admit(ffs_pool *p, const ffs_episode_desc *ep, int *slot_out
     zero(E.sums, sizeof(double) * 4);
     cp(p->d_eps + si, &E, sizeof(PoolEpisode));
     if (e != cudaSuccess) return undo(fail(FFS_ERR_CUDA, std::string("admission upload: ") + cudaGetErrorString(e)));
-    if ((e = launch_prepare_flags<2>(E.flags, E.wallmask, nullptr, 0u, d.nx, d.ny, 1, st)) != cudaSuccess)
+    if ((e = launch_prepare_flags<2>(E.flags, E.wallmask, nullptr, nullptr, 0u, d.nx, d.ny, 1, st)) != cudaSuccess)
         return undo(fail(FFS_ERR_CUDA, std::string("prepare flags: ") + cudaGetErrorString(e)));
     switch (p->d.storage) {
     case FFS_STORAGE_F32: r = init_episode<float>(p, s, d.boundary_velocities); break;

@@ -129,6 +129,7 @@ template <typename T> __device__ __forceinline__ GridArgs<T> episode_args(const 
     g.wall_stream = 0;
     g.feed = kBitOutletSrc;
     g.feeders = nullptr;
+    g.feeders_n = nullptr;
     g.feeders_cap = 0;
     g.omega = e.omega;
     g.codec = e.codec;

@@ -54,19 +54,35 @@ def test_d2q9_cuts(cuda, monkeypatch, nx, ny, rows, periodic):
 @pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
 def test_d2q9_cuts_round_identically(cuda, monkeypatch, storage):
     """A moving solid and outlets on four sides: the same bits for every cut."""
+    wl = W.swimmer_2d(nx=150, ny=70, body_frac=0.5, n_boundary=80, seed=3)
+    _same_bits(monkeypatch, wl, storage)
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("nx,ny,periodic", [(64, 32, False), (65, 33, True), (33, 9, False), (131, 75, False), (31, 7, True), (2, 3, False)])
+def test_tiles_and_march_round_identically(cuda, monkeypatch, nx, ny, periodic, storage):
+    """Walls and solids at random, an inlet and outlets, no surface."""
+    _same_bits(monkeypatch, _box2(nx, ny, periodic, nx + 2 * ny), storage)
+
+
+def _same_bits(monkeypatch, wl, storage):
+    """Tiles, then the march with several rows per unit."""
     import torch
 
-    wl = W.swimmer_2d(nx=150, ny=70, body_frac=0.5, n_boundary=80, seed=3)
     out = []
-    for rows in ("1", "5", "14"):
-        monkeypatch.setenv("FFS_MARCH_ROWS", rows)
+    for rows in (None, "1", "5", "14"):
+        if rows is None:
+            monkeypatch.delenv("FFS_MARCH_ROWS", raising=False)
+        else:
+            monkeypatch.setenv("FFS_MARCH_ROWS", rows)
         g, s = make_gpu(wl, storage)
         for k in range(6):
-            s.update(*wl.surface_at(k))
+            if s is not None:
+                s.update(*wl.surface_at(k))
             g.step(s)
         torch.cuda.synchronize()
         assert g.status() == 0
-        out.append((g.get_moments(), s.forces64.cpu().numpy()))
+        out.append((g.get_moments(), s.forces64.cpu().numpy() if s is not None else np.zeros(1)))
         g.close()
     for m, f in out[1:]:
         assert np.array_equal(out[0][0], m)
