@@ -27,11 +27,11 @@ FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3,-ffp-contrac
          "-I", CSRC, "-I", os.path.join(ROOT, "include")]
 
 
-# Per-file flags.  The kernels of the step are compiled without implicit
-# multiply-add contraction (every fused multiply-add in them is an explicit
-# one), so that kernels which differ only in register budget, scheduling and how
-# their work is cut up round identically: the cut that a grid's size or the
-# serving pool's mix picks cannot change a result.
+# Per-file flags.  The dense passes and the D2Q9 link cells are compiled without
+# implicit multiply-add contraction (every fused multiply-add in them is an
+# explicit one), so that kernels which differ only in register budget, scheduling
+# and how their work is cut up round identically: the cut that a grid's size or
+# the serving pool's mix picks cannot change a result.
 FILE_FLAGS = {f: ["-fmad=false"] for f in ("ffs_batch2d.cu", "ffs_dense2d.cu", "ffs_dense3d.cu", "ffs_links.cu")}
 
 

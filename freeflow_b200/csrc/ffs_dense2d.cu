@@ -12,8 +12,7 @@
 // Two options of the reference's own 2D kernel need populations as such: the
 // binary16 tile (ref_half_populations) and walls that stream
 // (ref_2d_wall_stream).  They, and grids whose moment indices do not fit in 32
-// bits, take dense2d_kernel: one CTA = one 32 x 8 tile, its populations plus a
-// one-cell halo in shared memory.
+// bits, take the kernel of ffs_ref2d.cu.
 #include <algorithm>
 #include <cstdlib>
 
@@ -28,13 +27,6 @@ namespace fflbm {
 // kernel spills 88 B around it, outside the row loop's common path); five (96
 // registers) spilled in the loop and ran the pool's pass 3 % slower, three 10 %.
 constexpr int kMarchWarps = 16;
-
-template <typename T, bool HALF>
-__global__ void __launch_bounds__(D2::kThreads) dense2d_kernel(GridArgs<T> g)
-{
-    __shared__ float sp[9][D2::kHY][D2::kHX];
-    dense2d_tile<T, HALF>(g, blockIdx.x * D2::kTX, blockIdx.y * D2::kTY, sp);
-}
 
 // Tile form of the march: one CTA = one 32 x 8 tile, a thread per cell.  The
 // deviations F' of the tile and the cells around it go through shared memory,
@@ -157,14 +149,7 @@ template <typename T> bool dense2d_detects(const GridArgs<T> &g)
 
 template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStream_t s, const DetectArgs *detect)
 {
-    if (!dense2d_detects(g)) {
-        dim3 grid((g.nx + D2::kTX - 1) / D2::kTX, (g.ny + D2::kTY - 1) / D2::kTY);
-        if (g.half_pops)
-            dense2d_kernel<T, true><<<grid, D2::kThreads, 0, s>>>(g);
-        else
-            dense2d_kernel<T, false><<<grid, D2::kThreads, 0, s>>>(g);
-        return cudaGetLastError();
-    }
+    if (!dense2d_detects(g)) return launch_ref2d<T>(g, s);
     const int sms = device_sms();
     const int lanes = detect ? detect_lanes2(detect->s.ne, sms) : 32;
     const long long detectors = detect ? std::min<long long>(((long long)detect->s.ne * lanes + 31) / 32, (long long)sms * 32) : 0; // warps

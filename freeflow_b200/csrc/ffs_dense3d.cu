@@ -36,7 +36,7 @@
 //   * moments are SoA planes in HBM (128 B coalesced per warp and moment);
 //     moments, flag bytes and wall masks are prefetched a plane ahead;
 //     outlets are fed by their inner neighbour in the same pass, and cells with
-//     moving-boundary links are left to the sparse link kernel (ffs_links.cu).
+//     moving-boundary links are left to the sparse link kernel (ffs_links_kernels.cuh).
 #include "ffs_dense2d.cuh"
 #include "ffs_dense3d.cuh"
 

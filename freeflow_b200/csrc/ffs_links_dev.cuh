@@ -1,5 +1,5 @@
 // Device bodies of the moving-boundary stages, shared by the single-grid
-// kernels (ffs_links.cu) and the batched many-grid kernels (ffs_batch2d.cu).
+// kernels (ffs_links_kernels.cuh) and the batched many-grid kernels (ffs_batch2d.cu).
 #pragma once
 #include "ffs_geom.cuh"
 #include "ffs_links.cuh"
@@ -581,7 +581,8 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
 // directions q, q + G, ...  As link_cell_update3, with every load of a lane's
 // directions issued before any is tested.  The raw moments are summed in the
 // same order for G = 4 and 16: (q, q + 8), then q + 4, then across lanes by 2
-// and by 1.
+// and by 1; every multiply-add here and in what it calls is explicit, or the
+// compiler would choose them for each G and the pool and a grid round apart.
 template <typename T, bool HALF, int G>
 __device__ __forceinline__ void link_cell_update2(const GridArgs<T> &g, const unsigned long long *links, uint32_t slot,
                                                   uint32_t cell, long long *acc, const SurfaceArgs &s,
@@ -641,14 +642,17 @@ __device__ __forceinline__ void link_cell_update2(const GridArgs<T> &g, const un
                                              geom::mul((float)(x - cx), cl), geom::mul((float)(y - cy), cl));
             if (!h.hit) continue;
             // wall velocity at the hit point, in lattice units
-            float uw[2];
+            float uw[2], a[2];
+            const float scale = sc.ct / sc.cl;
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
-                uw[k] = (s.U[(size_t)va * 2 + k] * h.b[0] + s.U[(size_t)vb * 2 + k] * h.b[1]) * (sc.ct / sc.cl);
+            for (int k = 0; k < 2; ++k) {
+                a[k] = fmaf(s.U[(size_t)va * 2 + k], h.b[0], s.U[(size_t)vb * 2 + k] * h.b[1]);
+                uw[k] = __fmul_rn(a[k], scale);
+            }
             // moving-wall population: Hermite expansion with the cell's density,
             // the wall velocity and pi' = pi + uw uw - u u
-            const float mw[6] = {mc[0], uw[0], uw[1], mc[3] + uw[0] * uw[0] - mc[1] * mc[1],
-                                 mc[4] + uw[1] * uw[1] - mc[2] * mc[2], mc[5] + uw[0] * uw[1] - mc[1] * mc[2]};
+            const float mw[6] = {mc[0], uw[0], uw[1], fmaf(-mc[1], mc[1], fmaf(uw[0], uw[0], mc[3])),
+                                 fmaf(-mc[2], mc[2], fmaf(uw[1], uw[1], mc[4])), fmaf(-mc[1], mc[2], fmaf(uw[0], uw[1], mc[5]))};
             Coef<2> wc;
             wc.make(mw);
             const float fout = wc.population(cx, cy, 0);
@@ -657,8 +661,8 @@ __device__ __forceinline__ void link_cell_update2(const GridArgs<T> &g, const un
             fin = fmaxf(fin, 0.0f);
             pop[t] = fout;
             // momentum exchange, lattice units: fin (-c - uw) - fout (c - uw)
-            const float Fx = fin * (-(float)cx - uw[0]) - fout * ((float)cx - uw[0]);
-            const float Fy = fin * (-(float)cy - uw[1]) - fout * ((float)cy - uw[1]);
+            const float Fx = fmaf(fin, fmaf(-a[0], scale, -(float)cx), -(fout * fmaf(-a[0], scale, (float)cx)));
+            const float Fy = fmaf(fin, fmaf(-a[1], scale, -(float)cy), -(fout * fmaf(-a[1], scale, (float)cy)));
             const uint32_t vert[3] = {va, vb, 0u};
             const float share[3][3] = {{Fx * h.b[0], Fy * h.b[0], 0.0f}, {Fx * h.b[1], Fy * h.b[1], 0.0f}, {0.0f, 0.0f, 0.0f}};
             add_forces_warp<2>(acc, true, e, vert, share, g.status);

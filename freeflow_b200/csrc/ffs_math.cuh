@@ -70,8 +70,8 @@ template <> struct Coef<2> {
         m1x = r3 * ux; m1y = r3 * uy;
         m2xx = r3 * pxx; m2yy = r3 * pyy; m2xy = 9.0f * r * pxy;
         float rux = r * ux, ruy = r * uy;
-        qxxy = 9.0f * fmaf(pxx, uy, 2.0f * ux * (pxy - rux * uy));
-        qxyy = 9.0f * fmaf(pyy, ux, 2.0f * uy * (pxy - ruy * ux));
+        qxxy = 9.0f * fmaf(pxx, uy, 2.0f * ux * fmaf(-rux, uy, pxy));
+        qxyy = 9.0f * fmaf(pyy, ux, 2.0f * uy * fmaf(-ruy, ux, pxy));
     }
     // all nine populations, reference numbering
     __device__ __forceinline__ void populations(float *f) const
@@ -101,8 +101,7 @@ template <> struct Coef<2> {
         s = fmaf(m2xx, gx, s); s = fmaf(m2yy, gy, s);
         s = fmaf(m2xy, fx * fy, s);
         s = fmaf(qxxy, gx * fy, s); s = fmaf(qxyy, fx * gy, s);
-        const float w = wgt2(cx + 1, cy + 1);
-        return w * s;
+        return __fmul_rn(wgt2(cx + 1, cy + 1), s);
     }
 };
 
@@ -324,13 +323,12 @@ __device__ __forceinline__ void collide2(const float *R, float omega, float *m)
     float ir = recip(rho);
     float ux = R[1] * ir, uy = R[2] * ir;
     float omw = 1.0f - omega;
-    float ux2 = ux * ux, uy2 = uy * uy;
-    float half_u2 = 0.5f * (ux2 + uy2);
-    float dev = 0.5f * (R[3] - R[4]) * omw * ir;
-    float an = 0.5f * omega * (ux2 - uy2);
+    float ux2 = ux * ux;
+    float half_u2 = 0.5f * fmaf(uy, uy, ux2), dif = fmaf(-uy, uy, ux2);
+    float dev = 0.5f * (R[3] - R[4]) * omw, half_om = 0.5f * omega;
     m[0] = rho; m[1] = ux; m[2] = uy;
-    m[3] = half_u2 + dev + an;
-    m[4] = half_u2 - dev - an;
+    m[3] = fmaf(half_om, dif, fmaf(dev, ir, half_u2));
+    m[4] = fmaf(-half_om, dif, fmaf(-dev, ir, half_u2));
     m[5] = fmaf(omw * R[5], ir, omega * ux * uy);
 }
 
