@@ -354,6 +354,14 @@ template <typename T> struct MomentPlanes {
 template <typename T> constexpr bool kRingWarps = !StorageTraits<T>::kEncoded;
 template <typename T> constexpr int kThreads3 = D3::kTile + (kRingWarps<T> ? 64 : 0);
 
+// The one barrier of a plane.  Tile and ring warps meet at it from different
+// places of the source, which __syncthreads() does not allow for; every warp
+// passes it ze - zb + 2 times.
+template <typename T> __device__ __forceinline__ void plane_barrier()
+{
+    asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(kThreads3<T>) : "memory");
+}
+
 // One CTA: 8 warps own the 32 x 8 tile's columns, and the ring warps, where
 // there are any, the 84 halo cells around it.
 // IDX32: every moment, flag and mask index (k * ncell + cell) fits in 32
@@ -436,7 +444,7 @@ __global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g,
                     store_row_paired<0>(coefficients(ra), buf, ca);
                 }
                 if (p < ze) load_cell(p + 1, oa, ra, ha);
-                __syncthreads(); // plane p is in buf; the tile has left the other buffer
+                plane_barrier<T>(); // plane p is in buf; the tile has left the other buffer
             }
         } else {
             const bool has = lane < 2 * D3::kHY, left = lane < D3::kHY;
@@ -459,7 +467,7 @@ __global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g,
                     }
                 }
                 if (p < ze) load_cell(p + 1, off, raw, h);
-                __syncthreads();
+                plane_barrier<T>();
             }
         }
         return;
@@ -583,7 +591,7 @@ __global__ void __launch_bounds__(kThreads3<T>, 2) dense3d_kernel(GridArgs<T> g,
         // of their own neighbours that must not trigger any work)
         const bool upd_n = is_updated(fn & kTypeMask) && !(fn & kBitLink);
         const uint32_t wn = (upd_n && (fn & (kBitNearWall | kBitOutletSrc))) ? g.wallmask[cell_at(p + 1)] : 0u;
-        __syncthreads();
+        plane_barrier<T>();
         if (inside) {
             constexpr uint32_t kWall = wall_bits_mask<3>();
             // the cell at z = p - 1 is complete: collide, store, feed outlets
