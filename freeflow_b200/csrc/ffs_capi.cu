@@ -754,10 +754,13 @@ ffs_status ffs_lbm_profile_read(ffs_lbm *h, ffs_profile *out, int reset)
 // the table has twice as many slots as the supported link cells, so it is at
 // most half full, like the table ffs_lbm_step sizes for itself):
 //   keys  [kNoallocSlots]  u32, 0 = empty slot          must start at 0
-//   list  [kNoallocSlots]  u32, claimed slots (one segment) no requirement
+//   list  [kNoallocSlots]  u32, claimed slots            no requirement
 //   count, done u32 (own 256-byte line)                  must start at 0
 //   links [kNoallocSlots * Q] u64, ~0 = no link          must start at ~0
 //   acc   [kNoallocMaxVertices * DIM] i64 force sums     must start at 0
+// The table counts its claims in one counter: the layout has no room for more,
+// and its size is documented.  On D2Q9 that is the faster form (kOneCounterCap);
+// a D3Q27 surface of n link cells waits about n ns longer in detection.
 // Every call clears all four on its stream before its first kernel, so a
 // call never depends on the previous one having finished cleanly.  Calls
 // that overlap in time on one device (two streams, two threads, two grids)

@@ -371,17 +371,12 @@ __device__ __forceinline__ void detect_elements2_warp(const GridArgs<T> &g, uint
 // share is first rounded to 2^-24 (as an int32) and then scaled by 2^8,
 // which is exactly what summing the int32 shares of a cell's links to one
 // element and scaling the sum would give; a share beyond +-127 lattice units
-// is clamped and flagged.  (An earlier form summed the links of one element
-// within the warp first, with __match_any_sync and __reduce_add_sync over
-// partial masks; the compiler loops such collectives per group, which cost
-// about 120 instructions per cell, more than the atomics they saved.)
+// is clamped and flagged.  (Summing the links of one element within the warp
+// first, with __match_any_sync and __reduce_add_sync over partial masks, took
+// about 120 instructions per cell, more than the atomics it saved.)
 template <int DIM>
-__device__ __forceinline__ void add_forces_warp(long long *acc, bool active, uint32_t elem, const uint32_t *vert,
-                                                const float (*share)[3], uint32_t *status, uint32_t group = 0)
+__device__ __forceinline__ void add_forces(long long *acc, const uint32_t *vert, const float (*share)[3], uint32_t *status)
 {
-    (void)elem;
-    (void)group;
-    if (!active) return;
 #pragma unroll
     for (int j = 0; j < DIM; ++j)
 #pragma unroll
@@ -418,7 +413,7 @@ constexpr int kPoolLinkGroup = 4;
 // calls this together (the force sums and the reduction are warp-wide); a
 // group with valid = false has no cell in this iteration and only takes part in
 // those, with arguments that still name a real cell.
-template <typename T, bool HALF>
+template <typename T>
 __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const unsigned long long *links,
                                                  uint32_t slot, uint32_t cell, long long *acc,
                                                  const SurfaceArgs &s, const StepScalars &sc, bool valid = true)
@@ -441,7 +436,6 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
     float mc[NM];
     float pop = 0.0f;
     bool has_share = false;
-    uint32_t hit_elem = 0xffffffffu;
     uint32_t vshare[3] = {0, 0, 0};
     float share[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}; // [vertex][component]
     // Every load the update may need goes out before any of them is tested:
@@ -475,7 +469,6 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
                 Coef<DIM> nc;
                 nc.make(mn);
                 float v = nc.population(cx, cy, cz);
-                if (HALF) v = round_half(v);
                 pulled = fmaxf(v, 0.0f);
             }
             bool done = false;
@@ -483,7 +476,6 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
             const bool bb = is_bounce_back<DIM>(fb & kTypeMask);
             if (bb) {
                 float v = own.population(-cx, -cy, -cz);
-                if (HALF) v = round_half(v);
                 pop = fmaxf(v, 0.0f);
                 done = true;
             } else if (notCross) {
@@ -521,7 +513,6 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
                         wc.make(mw);
                         const float fout = wc.population(cx, cy, cz);
                         float fin = own.population(-cx, -cy, -cz);
-                        if (HALF) fin = round_half(fin);
                         fin = fmaxf(fin, 0.0f);
                         pop = fout;
                         done = true;
@@ -531,7 +522,6 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
 #pragma unroll
                         for (int k = 0; k < DIM; ++k) F[k] = fin * (-c3[k] - uw[k]) - fout * (c3[k] - uw[k]);
                         has_share = true;
-                        hit_elem = e;
 #pragma unroll
                         for (int j = 0; j < DIM; ++j) {
                             vshare[j] = vv[j];
@@ -545,7 +535,7 @@ __device__ __forceinline__ void link_cell_update3(const GridArgs<T> &g, const un
         }
     }
     // forces: one share per (link, element vertex), summed per element
-    add_forces_warp<DIM>(acc, has_share, hit_elem, vshare, share, g.status, (threadIdx.x & 31) / G);
+    if (has_share) add_forces<DIM>(acc, vshare, share, g.status);
     // raw moments by reduction within the group (lanes Q.. add exact zeros,
     // so the sums equal those of a whole-warp reduction)
     int cx = 0, cy = 0, cz = 0;
@@ -665,7 +655,7 @@ __device__ __forceinline__ void link_cell_update2(const GridArgs<T> &g, const un
             const float Fy = fmaf(fin, fmaf(-a[1], scale, -(float)cy), -(fout * fmaf(-a[1], scale, (float)cy)));
             const uint32_t vert[3] = {va, vb, 0u};
             const float share[3][3] = {{Fx * h.b[0], Fy * h.b[0], 0.0f}, {Fx * h.b[1], Fy * h.b[1], 0.0f}, {0.0f, 0.0f, 0.0f}};
-            add_forces_warp<2>(acc, true, e, vert, share, g.status);
+            add_forces<2>(acc, vert, share, g.status);
         }
     }
     float R[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};

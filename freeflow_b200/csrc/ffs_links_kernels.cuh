@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256, DIM == 2 ? 2 : 5) link_cells_kernel(const
         const uint32_t slot = items.slot(lt, valid ? w + group : w);
         const uint32_t cell = lt.keys[slot] - 1;
         if constexpr (DIM == 2) link_cell_update2<T, HALF, G>(g, lt.links, slot, cell, lt.acc, s, sc, valid);
-        else link_cell_update3<T, HALF>(g, lt.links, slot, cell, lt.acc, s, sc, valid);
+        else link_cell_update3<T>(g, lt.links, slot, cell, lt.acc, s, sc, valid);
         // return the slot to the empty state and drop the cell's LINK bit
         for (int l = lane; valid && l < Q; l += G) lt.links[(size_t)slot * Q + l] = ~0ull;
         __syncwarp();

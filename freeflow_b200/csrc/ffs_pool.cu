@@ -226,7 +226,7 @@ int64_t mix_cells(const ffs_pool *p)
     return c;
 }
 
-// Fills the host active table for the current tile shape.
+// Fills the host active table for the current rows per unit.
 void build_active(ffs_pool *p)
 {
     PoolActive &A = *p->h_act;

@@ -47,7 +47,7 @@ struct PoolParams {
 };
 
 // The admitted episodes in admission order with prefix sums of their dense
-// tiles, elements and vertices.  Kernels read the count from device memory,
+// units, elements and vertices.  Kernels read the count from device memory,
 // so one captured graph serves every mix.
 struct PoolActive {
     uint32_t n;

@@ -13,7 +13,7 @@
  * A pool keeps every admitted episode's state on the device and advances all
  * of them by one control step with one CUDA-graph launch: per substep the
  * swimmer kinematics, link detection, the fused stream/collide pass (one
- * persistent launch over a packed list of tiles of all grids), the moving-
+ * persistent launch over a packed list of units of all grids), the moving-
  * wall link cells and the force reduction run once for the whole pool.
  * Outputs per control step (energy, mean force and torque, per-vertex
  * forces of the last substep, status) are reduced on the device.
@@ -90,15 +90,15 @@ typedef struct {
 typedef struct {
     int64_t budget_bytes, free_bytes, largest_free_bytes;
     int active_episodes;
-    int tiles;                 /* dense tiles per substep over all episodes */
-    int tile_x, tile_y;        /* tile shape in use (chosen by ffs_pool_tune) */
+    int tiles;                 /* units of the dense pass per substep over all episodes */
+    int tile_x, tile_y;        /* columns and rows of a unit (rows chosen by ffs_pool_tune) */
     int64_t advances;          /* control steps launched */
     int64_t graph_builds;      /* CUDA graphs instantiated */
     int64_t cells;             /* fluid cells over all admitted episodes */
     int64_t tuned_cells;       /* fluid cells of the mix at the last tuning */
     double dense_ms;           /* one dense pass over that mix (CUDA events, mean of 5) */
-    int strip;                 /* 1: the dense unit is a strip of tile_x columns and tile_y
-                                  rows walked row by row; 0: a tile_x x tile_y tile */
+    int strip;                 /* always 1: a unit is tile_x columns and tile_y rows walked row by row
+                                  (0 would be a tile; no such unit is left) */
     int pad;
 } ffs_pool_info;
 
@@ -125,7 +125,7 @@ ffs_status ffs_pool_set_action(ffs_pool *pool, int slot, const float *actions, i
 ffs_status ffs_pool_set_actions(ffs_pool *pool, int n, const int *slots, const float *actions);
 
 /* Launches one control step of every admitted episode; returns without
- * waiting.  The first call after the mix changed re-uploads the tile table;
+ * waiting.  The first call after the mix changed re-uploads the unit table;
  * the first call (and ffs_pool_tune) builds the CUDA graph.  The pinned
  * parameter and output buffers are double-buffered, so the call does not
  * wait for the previous control step: it waits only while the step before
@@ -143,11 +143,13 @@ ffs_status ffs_pool_collect(ffs_pool *pool, int slot, ffs_pool_output *out, doub
 ffs_status ffs_pool_collect_many(ffs_pool *pool, int n, const int *slots, ffs_pool_output *out);
 
 /* Current moments of the slot in the reference AoS layout (nx*ny*6 floats,
- * host memory); synchronous.  For tests and inspection. */
+ * host memory); synchronous.  For tests and inspection.  The first call (and
+ * one for a larger episode) allocates nx*ny*24 bytes of device memory outside
+ * budget_bytes, which the pool keeps until it is destroyed. */
 ffs_status ffs_pool_get_moments(ffs_pool *pool, int slot, float *moments);
 
-/* Times the candidate tile shapes of the dense pass on the current mix and
- * keeps the fastest (a project autotuner; rebuilds the graph). */
+/* Times the candidate numbers of rows per unit of the dense pass on the current
+ * mix and keeps the fastest (a project autotuner; rebuilds the graph). */
 ffs_status ffs_pool_tune(ffs_pool *pool);
 
 ffs_status ffs_pool_get_info(const ffs_pool *pool, ffs_pool_info *info);
