@@ -40,6 +40,7 @@
 #include "ffs_dense2d.cuh"
 #include "ffs_dense3d.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
@@ -166,7 +167,7 @@ __device__ __forceinline__ void slice_sums_paired(const float *buf, int c_own, f
     Sm[5] = fmaf(0.25f, X2m[2] + X2m[0], X2m[1]);
 }
 
-// The z level of Coef3V::populations_each (the Hermite sums over c_z of the
+// The z level of the expansion (the Hermite sums over c_z of the
 // six coefficient groups), with the c_z = -1 / +1 entries as pairs (p) and
 // the c_z = 0 entry apart (m): herm3v gives ((a0 + a2) - a1, fma(-1/2, a2,
 // a0), (a0 + a2) + a1), herm2v (a0 - a1, a0, a0 + a1).
@@ -194,7 +195,7 @@ struct ZLevel {
 };
 
 // All 27 unweighted populations of one cell into the paired layout: the y and
-// x levels of populations_each, paired over c_z = -1 / +1.
+// x levels of the expansion, paired over c_z = -1 / +1.
 __device__ __forceinline__ void store_populations_paired(const Coef3V<float> &c, float *buf, int cell)
 {
     const ZLevel z(c);
@@ -217,7 +218,7 @@ __device__ __forceinline__ void store_populations_paired(const Coef3V<float> &c,
     }
 }
 
-// The 9 populations with c_y = KY - 1 of a halo row cell (populations_row)
+// The 9 populations with c_y = KY - 1 of a halo row cell
 // into the paired layout.
 template <int KY> __device__ __forceinline__ void store_row_paired(const Coef3V<float> &c, float *buf, int cell)
 {
@@ -250,7 +251,7 @@ template <int KY> __device__ __forceinline__ void store_row_paired(const Coef3V<
     for (int kx = 0; kx < 3; ++kx) store_pair(buf, (kx + 3 * KY) * kHalo + cell, Fp[kx], Fm[kx]);
 }
 
-// The 9 populations with c_x = sx of a halo column cell (populations_col)
+// The 9 populations with c_x = sx of a halo column cell
 // into the paired layout; kx = sx + 1.
 __device__ __forceinline__ void store_col_paired(const Coef3V<float> &c, float sx, int kx, float *buf, int cell)
 {
@@ -704,6 +705,8 @@ template <typename T, bool IDX32, bool FEED> static cudaError_t launch_as(const 
     int tx = (g.nx + kTX - 1) / kTX, ty = (g.ny + kTY - 1) / kTY;
     int nchunk = choose_zchunks(tx * ty, g.nz, slots);
     int zchunk = (g.nz + nchunk - 1) / nchunk;
+    // FFS_DENSE3D_PLANES pins the planes per chunk (tests run several cuts)
+    if (const char *planes = std::getenv("FFS_DENSE3D_PLANES")) zchunk = std::max(1, std::min(g.nz, std::atoi(planes)));
     dim3 grid(tx, ty, (g.nz + zchunk - 1) / zchunk);
     MomentPlanes<T> mp;
     for (int k = 0; k < 10; ++k) {

@@ -1,11 +1,8 @@
-"""Every D3Q27 dense-kernel variant against the oracle (the tuner picks one
-per grid by speed, so each must pass the parity cases on its own).
-
-Variants: 0 and 1 are the single-plane z-march built for two and three CTAs
-per SM; 2 is the two-CTA march with the paired shared-memory layout and
-packed c_z = -1 / +1 arithmetic; 3 is variant 2 with each halo plane's
-moments staged in shared memory by TMA copies (32-bit indices only; grids
-whose rows are not a multiple of 16 bytes run variant 2).
+"""The D3Q27 dense pass against the oracle, with 32-bit indices (grids of up to
+429 M cells) and 64-bit ones (forced by FFS_DENSE3D_INDEX64), and cut into
+chunks of planes at the depths where a cut can go wrong (FFS_DENSE3D_PLANES
+pins the planes per chunk that a grid's size would choose).  FP32 grids take the
+halo ring on two warps of its own, 16-bit ones on the tile's threads.
 Tolerances are those of test_gpu_parity.py: 2e-6 against the ref32 oracle,
 4e-6 next to walls (bounce-back added as a correction), 5e-6 against FP64.
 """
@@ -14,26 +11,19 @@ import pytest
 
 from freeflow_b200 import workloads as W
 
-from helpers import max_abs, run_pair
+from helpers import make_gpu, max_abs, run_pair
 
 pytestmark = pytest.mark.gpu
 
-# (variant, index width): the single-plane variants run with 32-bit indices on
-# grids of up to 429 M cells and 64-bit ones beyond; FFS_DENSE3D_INDEX64 forces
-# the 64-bit path here
-VARIANTS = [(0, 32), (1, 32), (2, 32), (3, 32), (0, 64), (1, 64), (2, 64)]
 
-
-@pytest.fixture(params=VARIANTS, ids=lambda v: f"v{v[0]}-i{v[1]}")
-def variant(request, monkeypatch):
-    v, width = request.param
-    monkeypatch.setenv("FFS_DENSE3D_VARIANT", str(v))
-    if width == 64:
+@pytest.fixture(params=[32, 64], ids=lambda w: f"i{w}")
+def index_width(request, monkeypatch):
+    if request.param == 64:
         monkeypatch.setenv("FFS_DENSE3D_INDEX64", "1")
-    return v
+    return request.param
 
 
-def test_swimmer(cuda, variant):
+def test_swimmer(cuda, index_width):
     wl = W.swimmer_3d(nx=64, ny=32, nz=32, body_frac=0.3, nlat=12, nlon=16, seed=5)
     gm, om, gf, of, st = run_pair(wl, 6)
     assert st == 0
@@ -41,14 +31,14 @@ def test_swimmer(cuda, variant):
     assert max_abs(gf, of) <= 1e-4 * np.abs(of).max()
 
 
-def test_taylor_green_periodic_vs_fp64(cuda, variant):
+def test_taylor_green_periodic_vs_fp64(cuda, index_width):
     wl = W.taylor_green_3d(n=32, u0=0.04, viscosity=0.005)
     gm, om, _, _, st = run_pair(wl, 20, precision="phys64")
     assert st == 0
     assert max_abs(gm, om) <= 5e-6
 
 
-def test_reference_halo(cuda, variant):
+def test_reference_halo(cuda, index_width):
     """Non-periodic faces: the halo wraps at the low and clamps at the high face."""
     wl = W.taylor_green_3d(n=20, u0=0.04, viscosity=0.01)
     gm, om, _, _, st = run_pair(wl, 8, periodic=0)
@@ -56,7 +46,7 @@ def test_reference_halo(cuda, variant):
     assert max_abs(gm, om) <= 2e-6
 
 
-def test_walls_inlet_outlet(cuda, variant):
+def test_walls_inlet_outlet(cuda, index_width):
     wl = W.swimmer_3d(nx=40, ny=24, nz=24, nlat=8, nlon=12)
     wl.elements = None
     gm, om, _, _, st = run_pair(wl, 8)
@@ -64,7 +54,7 @@ def test_walls_inlet_outlet(cuda, variant):
     assert max_abs(gm, om) <= 4e-6
 
 
-def test_open_face_with_wall_across_the_wrap(cuda, variant):
+def test_open_face_with_wall_across_the_wrap(cuda, index_width):
     wl = W.taylor_green_3d(n=20, u0=0.03, viscosity=0.01)
     f = wl.flags.reshape(20, 20, 20)
     f[:, :, 19] = W.WALL
@@ -76,7 +66,7 @@ def test_open_face_with_wall_across_the_wrap(cuda, variant):
 
 
 @pytest.mark.parametrize("nz", [17, 40])
-def test_odd_and_chunked_depths(cuda, variant, nz):
+def test_odd_and_chunked_depths(cuda, index_width, nz):
     """Plane counts that leave a single plane in the last pair, and depths
     split into several z chunks."""
     wl = W.swimmer_3d(nx=48, ny=24, nz=nz, body_frac=0.3, nlat=8, nlon=12, seed=9)
@@ -85,7 +75,7 @@ def test_odd_and_chunked_depths(cuda, variant, nz):
     assert max_abs(gm, om) <= 4e-6
 
 
-def test_periodic_width_not_a_tile_multiple(cuda, variant):
+def test_periodic_width_not_a_tile_multiple(cuda, index_width):
     """nx = 48 with x periodic: the last tile's halo wraps onto the first
     columns, and its cells beyond nx only serve as halo."""
     wl = W.taylor_green_3d(n=48, u0=0.04, viscosity=0.01)
@@ -98,7 +88,7 @@ def test_periodic_width_not_a_tile_multiple(cuda, variant):
     assert max_abs(gm, om) <= 2e-6
 
 
-def test_odd_width(cuda, variant):
+def test_odd_width(cuda, index_width):
     """nx odd: rows whose cells do not pair up on 8-byte boundaries."""
     wl = W.swimmer_3d(nx=41, ny=24, nz=20, body_frac=0.3, nlat=8, nlon=12, seed=11)
     gm, om, _, _, st = run_pair(wl, 4)
@@ -106,19 +96,21 @@ def test_odd_width(cuda, variant):
     assert max_abs(gm, om) <= 4e-6
 
 
-@pytest.mark.parametrize("storage", ["f32", "f16"])
-def test_tuned_variants_round_identically(cuda, monkeypatch, storage):
-    """The first step's timing chooses among the variants, so all must give
-    the same bits (moments and surface forces, with walls, an inlet, an
-    outlet and a moving surface): the choice cannot change a result."""
+@pytest.mark.parametrize("storage", ["f32", "f16", "bf16"])
+@pytest.mark.parametrize("nx,ny,nz", [(64, 32, 32), (45, 27, 23)])
+def test_cuts_round_identically(cuda, monkeypatch, nx, ny, nz, storage):
+    """The same bits (moments and surface forces, with walls, an inlet, an outlet
+    and a moving surface) for every depth of a chunk and both index widths: the
+    cut that a grid's size picks cannot change a result."""
     import torch
 
-    from helpers import make_gpu
-
-    wl = W.swimmer_3d(nx=64, ny=32, nz=32, body_frac=0.4, nlat=16, nlon=24, seed=4)
+    wl = W.swimmer_3d(nx=nx, ny=ny, nz=nz, body_frac=0.4, nlat=16, nlon=24, seed=4)
     out = []
-    for v in ("0", "1", "2", "3"):
-        monkeypatch.setenv("FFS_DENSE3D_VARIANT", v)
+    for planes, wide in [(None, False), (1, False), (5, False), (nz, False), (None, True), (7, True)]:
+        monkeypatch.delenv("FFS_DENSE3D_PLANES", raising=False)
+        monkeypatch.setenv("FFS_DENSE3D_INDEX64", "1" if wide else "0")
+        if planes:
+            monkeypatch.setenv("FFS_DENSE3D_PLANES", str(planes))
         g, s = make_gpu(wl, storage)
         for k in range(6):
             s.update(*wl.surface_at(k))
@@ -130,3 +122,14 @@ def test_tuned_variants_round_identically(cuda, monkeypatch, storage):
     for o in out[1:]:
         assert np.array_equal(out[0][0], o[0])
         assert np.array_equal(out[0][1], o[1])
+
+
+@pytest.mark.parametrize("planes", [1, 4, 19])
+def test_cuts_random_node_types(cuda, monkeypatch, planes):
+    """Walls, solids and moving-solid cells at random against the oracle, chunk by chunk."""
+    from test_gpu_random_flags import _workload_3d
+
+    monkeypatch.setenv("FFS_DENSE3D_PLANES", str(planes))
+    gm, om, _, _, st = run_pair(_workload_3d(37, 21, 19, False, seed=5), 5)
+    assert st == 0
+    assert max_abs(gm, om) <= 4e-6

@@ -1,6 +1,6 @@
 """ffs_lbm_step inside a CUDA graph.
 
-After one eager step (which picks the dense-kernel variant and sizes the link
+After one eager step (which sizes the link
 table), the step records only stream work: kernel launches and the events that
 fork link detection onto the grid's side stream and join it back.  A graph
 captured on the caller's stream then replays like eager steps.  The grid's

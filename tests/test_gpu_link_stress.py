@@ -40,12 +40,10 @@ def _links(wl):
     return gcq, gkey, ocq, okey
 
 
-@pytest.mark.parametrize("seed", [0, 1, 2])
-def test_random_segments_links_identical(cuda, seed):
+def _random_segments(seed, n=400):
     rng = np.random.default_rng(seed)
     wl = W.cylinder_channel_2d(nx=96, ny=64, radius=6.0, center=(30.0, 30.0), nseg=32, seed=seed)
     cl = wl.fluid_dx
-    n = 400
     c = rng.uniform([4, 4], [wl.nx - 5, wl.ny - 5], size=(n, 2)) * cl
     ang = rng.uniform(0, 2 * math.pi, n)
     special = rng.random(n) < 0.3     # axis-aligned and diagonal segments
@@ -55,10 +53,45 @@ def test_random_segments_links_identical(cuda, seed):
     a, b = _snap(c - d, rng, cl), _snap(c + d, rng, cl)
     wl.rest = np.concatenate([a, b]).astype(np.float32)
     wl.elements = np.stack([np.arange(n), np.arange(n) + n], 1).astype(np.uint32)
-    gcq, gkey, ocq, okey = _links(wl)
+    return wl
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_random_segments_links_identical(cuda, seed):
+    gcq, gkey, ocq, okey = _links(_random_segments(seed))
     assert len(ocq) > 1000
     assert np.array_equal(gcq, ocq)
     assert np.array_equal(gkey, okey)
+
+
+@pytest.mark.parametrize("n", [400, 2600])
+@pytest.mark.parametrize("rows", [None, 6], ids=["tiles", "march"])
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_step_finds_the_same_links(cuda, monkeypatch, storage, rows, n):
+    """The step detects 2D links in CTAs of the dense pass's launch, with 32 or
+    (2,600 segments) 8 lanes a segment; debug_links and serial stage timing
+    launch detection by itself.  One step must give the same bits both ways:
+    every link enters moments and forces."""
+    import torch
+
+    if rows:
+        monkeypatch.setenv("FFS_MARCH_ROWS", str(rows))
+    wl = _random_segments(5, n)
+    v, u = wl.surface_at(0)
+    u = np.random.default_rng(7).uniform(-0.05, 0.05, v.shape).astype(np.float32) * np.float32(wl.fluid_dx / wl.dt)
+    out = []
+    for serial in (True, False):
+        g, surf = make_gpu(wl, storage)
+        if serial:
+            g.profile(True, serial=True)
+        surf.update(v, u)
+        g.step(surf)
+        torch.cuda.synchronize()
+        out.append((g.get_moments(), surf.forces64.cpu().numpy().copy()))
+        g.close()
+    assert np.abs(out[0][1]).max() > 0
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
 
 
 @pytest.mark.parametrize("seed", [0, 1])

@@ -1,9 +1,9 @@
 """Dense passes under random node types: grids of odd sizes (no dimension a
 multiple of the tile) with walls, static solids and moving-solid cells
 scattered through the interior and over the faces, an inlet and an outlet,
-with and without periodic axes, and random equilibrium states.  Every
-D3Q27 variant and the D2Q9 pass must match the oracle within the wall
-tolerance of test_gpu_parity.py (4e-6: near-wall cells add the bounce-back
+with and without periodic axes, and random equilibrium states.  The D3Q27
+pass (32- and 64-bit indices) and the D2Q9 pass (tiles and the row march) must
+match the oracle within the wall tolerance of test_gpu_parity.py (4e-6: near-wall cells add the bounce-back
 populations as a correction of the pulled ones)."""
 import numpy as np
 import pytest
@@ -53,30 +53,34 @@ def _workload_3d(nx, ny, nz, periodic, seed):
     return wl
 
 
-@pytest.fixture(params=[0, 1, 2, 3], ids=lambda v: f"v{v}")
-def variant(request, monkeypatch):
-    monkeypatch.setenv("FFS_DENSE3D_VARIANT", str(request.param))
+@pytest.fixture(params=[32, 64], ids=lambda w: f"i{w}")
+def index_width(request, monkeypatch):
+    if request.param == 64:
+        monkeypatch.setenv("FFS_DENSE3D_INDEX64", "1")
     return request.param
 
 
 @pytest.mark.parametrize("periodic", [False, True], ids=["open", "periodic"])
-def test_d3q27_random_node_types(cuda, variant, periodic):
+def test_d3q27_random_node_types(cuda, index_width, periodic):
     wl = _workload_3d(37, 21, 19, periodic, seed=3 + periodic)
     gm, om, _, _, st = run_pair(wl, 6)
     assert st == 0
     assert np.abs(gm - om).max() <= 4e-6
 
 
-def test_d3q27_random_node_types_multiple_of_16_width(cuda, variant):
-    """nx a multiple of 4 and 8, so that variant 3 stages by TMA (other widths fall back)."""
+def test_d3q27_random_node_types_multiple_of_16_width(cuda, index_width):
+    """nx a multiple of 16: the last tile in x is half outside the grid."""
     wl = _workload_3d(48, 21, 19, False, seed=7)
     gm, om, _, _, st = run_pair(wl, 6)
     assert st == 0
     assert np.abs(gm - om).max() <= 4e-6
 
 
+@pytest.mark.parametrize("rows", [None, 5], ids=["tiles", "march"])
 @pytest.mark.parametrize("periodic", [False, True], ids=["open", "periodic"])
-def test_d2q9_random_node_types(cuda, periodic):
+def test_d2q9_random_node_types(cuda, monkeypatch, periodic, rows):
+    if rows:
+        monkeypatch.setenv("FFS_MARCH_ROWS", str(rows))
     rng = np.random.default_rng(11 + periodic)
     wl = W.cylinder_channel_2d(nx=83, ny=45, nseg=16)
     wl.elements = None

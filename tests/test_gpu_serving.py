@@ -8,8 +8,8 @@
   * FP16 storage vs the FP64 oracle: relative L2 velocity error <= 1e-3
     (closed tank; FP32 storage, for scale, <= 5e-4)
   * admission by device memory, eviction, and graph reuse across mixes
-The identity tests run once per dense work unit (FFS_POOL_SHAPE pins it): the
-five tile shapes and the three row-marching strips must all give the same bits.
+The identity tests run once per number of rows in a unit of the dense pass
+(FFS_POOL_SHAPE pins it): all must give the same bits.
 """
 import numpy as np
 import pytest
@@ -20,7 +20,7 @@ from helpers import max_abs
 
 pytestmark = pytest.mark.gpu
 
-TILES, STRIPS = [0, 1, 2, 3, 4], [5, 6, 7]
+SHAPES = list(range(8))  # 1, 2, 3, 4, 6, 8, 11 and 14 rows a unit
 
 
 @pytest.fixture
@@ -47,7 +47,7 @@ def _run_pool(pool, slots_specs, control_steps):
     return outs
 
 
-@pytest.mark.parametrize("shape,storage", [(s, "f32") for s in TILES + STRIPS] + [(1, "f16"), (6, "f16"), (6, "bf16")])
+@pytest.mark.parametrize("shape,storage", [(s, "f32") for s in SHAPES] + [(1, "f16"), (6, "f16"), (6, "bf16")])
 def test_pool_f32_matches_single_grid_step(cuda, pin_shape, shape, storage):
     """Pool episodes against single grids of the same storage (FP32, and the
     16-bit paths with their codec), unit by unit: identical bits."""
@@ -68,7 +68,7 @@ def test_pool_f32_matches_single_grid_step(cuda, pin_shape, shape, storage):
     pool.close()
 
 
-@pytest.mark.parametrize("shape", [1] + STRIPS)
+@pytest.mark.parametrize("shape", [1, 5, 6, 7])
 def test_pool_matches_oracle(cuda, pin_shape, shape):
     from oracle.oracle import Oracle
 
@@ -100,10 +100,10 @@ def test_pool_matches_oracle(cuda, pin_shape, shape):
 
 
 @pytest.mark.parametrize("storage", ["f16", "f32"])
-def test_strip_and_tile_units_agree_on_odd_widths(cuda, pin_shape, storage):
-    """Odd row widths: 2-byte moments cannot be staged two per 4-byte copy, so
-    the strip kernel copies them one by one; walls on every side exercise the
-    bounce-back path of the strip kernel too."""
+def test_units_agree_on_odd_widths(cuda, pin_shape, storage):
+    """Odd row widths: a lane's two cells are not on a boundary of the pair and
+    are fetched one by one; walls on every side exercise the bounce-back path
+    too."""
     res = []
     for sides in ("outlets", "walls"):
         sp = S.make_episode(255, 131, seed=51, length=10, sides=sides)
@@ -123,7 +123,7 @@ def test_strip_and_tile_units_agree_on_odd_widths(cuda, pin_shape, storage):
             assert np.array_equal(ma, mb)
 
 
-@pytest.mark.parametrize("shape", [1] + STRIPS)
+@pytest.mark.parametrize("shape", [1, 5, 6, 7])
 def test_episode_alone_and_in_mix_identical(cuda, pin_shape, shape):
     pin_shape(shape)
     target = S.make_episode(512, 192, seed=31, length=10)
