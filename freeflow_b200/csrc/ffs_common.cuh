@@ -275,10 +275,12 @@ __device__ __forceinline__ uint32_t vel_dither(size_t idx, float rho)
 }
 // Two floats rounded to binary16 stochastically (lo in the low half), in one
 // conversion instruction: bits 0..12 of `r` decide the low value, bits 16..28
-// the high one, and a value rounds up in magnitude with probability (dropped
-// bits) / 2^13.  (The integer sequence this replaces, add 10 random bits and
-// truncate with the ends of binary16's range handled apart, took about seven
-// instructions per velocity.)
+// the high one, and a value rounds up in magnitude with the probability of its
+// distance from the lower neighbour, to within 2^-13 of their spacing.  That
+// holds for subnormal results too, whose spacing is 2^-24 (u * su below 2^-14:
+// the flow near rest).  (The integer sequence this replaces took about seven
+// instructions per velocity; it used 10 random bits and rounded that range to
+// nearest.)
 __device__ __forceinline__ uint32_t half2_sr(float lo, float hi, uint32_t r)
 {
     uint32_t d;
@@ -359,18 +361,6 @@ __device__ __forceinline__ void encode_store_strided(const float *m, T *base, si
     for (int k = 0; k < Lattice<DIM>::NM; ++k) base[idx + k * stride] = enc[k];
 }
 
-// Same as encode_store with planes[k] = base + k * stride and a 32-bit index
-// idx + k * stride (the caller guarantees it fits).
-template <int DIM, typename T>
-__device__ __forceinline__ void encode_store_idx32(const float *m, T *base, uint32_t idx, uint32_t stride,
-                                                   const Codec &c)
-{
-    T enc[Lattice<DIM>::NM];
-    encode_values<DIM, T>(m, idx, c, enc);
-#pragma unroll
-    for (int k = 0; k < Lattice<DIM>::NM; ++k) base[idx + (uint32_t)k * stride] = enc[k];
-}
-
 // The values encode_store writes for cell idx, as they read back: m itself
 // for FP32, the decoded rounded deviations otherwise.
 template <int DIM, typename T>
@@ -417,23 +407,6 @@ inline int device_sms()
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
     return n;
 }
-
-// cp.async (LDGSTS): 4-byte global -> shared copies that hold no registers
-// while in flight.  Both addresses must be 4-byte aligned.
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(src) : "memory");
-}
-// 16-byte copy (L2 only); both addresses must be 16-byte aligned.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// waits until at most N of this thread's committed groups are still in flight
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // Programmatic dependent launch: the kernel is scheduled while its predecessor
 // in the stream still runs (once every block of that one has started), and
