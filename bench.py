@@ -60,8 +60,8 @@ FALLBACK_HBM_GBS = 6650.0
 # (dram__bytes_read.sum + dram__bytes_write.sum), scaled to a launch by the
 # cells it processes; the capture and its command are in the named profile.
 DENSE_TRAFFIC_PER_CELL = {
-    (3, "f32"): (75.20, "profiles/dense3d_link_kernels_D3Q27_256x128x128_swimmer_f32.md"),
-    (3, "f16"): (35.98, "profiles/dense3d_D3Q27_256x128x128_swimmer_f16.md"),
+    (3, "f32"): (74.60, "profiles/dense3d_D3Q27_256x128x128_swimmer.md"),
+    (3, "f16"): (35.80, "profiles/dense3d_D3Q27_256x128x128_swimmer.md"),
 }
 
 
@@ -786,7 +786,7 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": traffic, "traffic_source": traffic_src,
                          "peak_kind": peak_kind,
-                         "kernel": "dense3d_kernel" if wl.dim == 3 else "dense2d_kernel",
+                         "kernel": "dense3d_kernel" if wl.dim == 3 else "tile2d_kernel",
                          "bytes_per_cell": bpc, "kernel_ms": round(dense_ms / max(1, dense_n), 4)},
             "stages_ms_per_step": {k: round(v[0] / max(1, v[1]), 4) for k, v in prof.items() if v[1]},
             "stages_alone_ms_per_step": stages_alone,

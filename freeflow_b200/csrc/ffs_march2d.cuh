@@ -16,7 +16,7 @@
 //
 // What bounds it: instruction issue, then HBM.  The tile-and-strip kernels it
 // replaced in the pool staged populations in shared memory and spent about 347
-// thread instructions per cell; the packed march takes 189 (FP16 serving mix,
+// thread instructions per cell; the packed march takes 191 (FP16 serving mix,
 // 14 rows, with detection).
 //
 // Bounce-back: a wall or solid cell is reconstructed from a zero state, so
