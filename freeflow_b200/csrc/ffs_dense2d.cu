@@ -24,8 +24,8 @@ namespace fflbm {
 
 // March warps (one-warp CTAs) per SM that the register budget is cut for: four
 // per scheduler leave 128 registers, which the march fills (the pool's FP32
-// kernel spills 88 B around it, outside the row loop's common path); five (96
-// registers) spilled in the loop and ran the pool's pass 3 % slower, three 10 %.
+// kernel spills 88 B, the 16-bit ones 4); five (96 registers) ran the pool's pass
+// 3 % slower, three 10 %.
 constexpr int kMarchWarps = 16;
 
 // Tile form of the march: one CTA = one 32 x 8 tile, a thread per cell.  The

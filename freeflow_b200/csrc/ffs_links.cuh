@@ -79,10 +79,9 @@ template <typename T> bool dense2d_detects(const GridArgs<T> &g);
 
 // Lanes per segment in the 2D detection of one surface.  Where every segment
 // can have a warp that is resident at once, 32: a warp's time is then its
-// chain of table insertions, which four lanes per direction share (ten steps
-// on 1200 x 400 with 198 segments: 257 us in FP32, against 274 with 8 lanes;
-// 229 against 227 in FP16).  Otherwise 8, which take a quarter of the
-// instructions.
+// chain of table insertions, which four lanes per direction share (a step on
+// 300 x 181 with 198 segments: 16.0 us in FP32, against 17.3 with 8 lanes; on
+// 160 x 96 the same).  Otherwise 8, which take a quarter of the instructions.
 inline int detect_lanes2(long long segments, int sms) { return segments <= 16ll * sms ? 32 : 8; }
 template <typename T> cudaError_t launch_dense2d(const GridArgs<T> &g, cudaStream_t s, const DetectArgs *detect = nullptr);
 

@@ -6,8 +6,9 @@
 // inner neighbour p = q - n (a Fluid node) when that velocity points outward,
 // and sets pi_nn = u_n(p)^2, in place on the freshly written buffer.  Each
 // outlet has exactly one feeder p, so the same writes are issued here once p's
-// new moments are final, straight into the buffer being written.  No other node reads q's entries
-// of that buffer during the step, so the result is the reference's.
+// new moments are final, straight into the buffer being written.  No other node
+// reads q's entries of that buffer during the step, so the result is the
+// reference's.
 #pragma once
 #include <type_traits>
 
@@ -109,10 +110,11 @@ __device__ __noinline__ void mark_outlets(uint32_t *flag_words, const uint32_t *
     }
 }
 
-// Outlets fed by cell p (mask word `word`), whose new moments are in g.dst, in one body for all
-// rules: this code is met cold, and a copy per rule took longer to fetch than
-// to run.  Link cells are left out: by their LINK bit, or with flag_words (bits
-// are on their way out) by the marks of their outlet nodes, which are taken off.
+// Outlets fed by cell p (mask word `word`), whose new moments are in g.dst, in
+// one body for all rules: this code is met cold, and a copy per rule took longer
+// to fetch than to run.  Link cells are left out: by their LINK bit, or with
+// flag_words (bits are on their way out) by the marks of their outlet nodes,
+// which are taken off.
 template <int DIM, typename T>
 __device__ __forceinline__ void feed_cell(const GridArgs<T> &g, uint32_t p, uint32_t word, uint32_t *flag_words)
 {
@@ -166,8 +168,9 @@ __device__ __noinline__ void feed_scan(const GridArgs<T> &g, uint32_t *flag_word
 }
 
 // Feeds the outlets of the grid's n = *g.feeders_n feeders but the link cells,
-// by warps `warp` of `nwarps`.  The list of feeders was made when the node types were
-// set; finding them in the flag bytes took 1 us of a 17 us step on 800 x 300.
+// by warps `warp` of `nwarps`.  The list of feeders was made when the node types
+// were set; finding them in the flag bytes took 1 us of a 17 us step on
+// 800 x 300.
 template <int DIM, typename T>
 __device__ __noinline__ void feed_pass(const GridArgs<T> &g, uint32_t n, uint32_t *flag_words, uint32_t warp, uint32_t nwarps)
 {
